@@ -207,17 +207,12 @@ struct LinearVisitor {
     };
     static cudaError_t prepare(const Sched &, const WsLayout &, cudaStream_t) { return cudaSuccess; }
     static cudaError_t finalize(const Sched &, const WsLayout &, cudaStream_t) { return cudaSuccess; }
-    // Resident CTAs per SM: the reverse worker fits 64 registers with 20 bytes of
-    // spills (8 CTAs: -3 % time per Riemann3 200^3 call against 6 at 80
-    // registers), the forward one 72 registers (7 CTAs).
-    static constexpr int kMinCtas = SIZE == 256 ? 4 : (FWD ? 7 : 8);
-    // A linear solve is usually one large instance: its epochs (~15 k tiles at
-    // 200^3) are published in batches; the worker's registers stay within the
-    // kMinCtas budget.
-    static constexpr bool kBulkPublish = true;
-    static constexpr bool kBatchScheduling = false;
+    // A linear solve is one instance and runs in rounds, a warp per tile.
+    static constexpr bool kQueueless = true;
+    static constexpr int kMinCtas = 1, kRoundG = 1, kRoundWarps = SIZE == 256 ? 8 : 16, kRoundCtas = 2;
+    using RoundSmem = Smem;
 
-    __device__ static void visit(const Sched &S, const Args &A, int t, int ii, int e, int lane, Smem &sm) {
+    __device__ static bool visit_round(const Sched &S, const Args &A, int t, int ii, int e, int lane, int, Smem &sm) {
         const Inst &I = S.inst[ii];
         const int n_o = t - I.tile_base;
         const long long base = (long long)n_o * SIZE;
@@ -344,7 +339,7 @@ struct LinearVisitor {
                 break;
             }
         }
-        bool self = !settled;
+        bool pushed = false;
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             const int n_i = lane + 32 * p;
@@ -356,8 +351,9 @@ struct LinearVisitor {
             if constexpr (FWD) {
                 for (int j = r0[p]; j < r1[p]; ++j) {  // the points that depend on this one
                     const int ty = __ldg(A.src + j) / SIZE;
-                    if (ty == n_o) self = true;
-                    else push_tile<false>(S, I, ii, I.tile_base + ty, e);
+                    if (ty == n_o) continue;
+                    push_round(S, I.tile_base + ty, e);
+                    pushed = true;
                 }
             } else {
                 for (int k = 0; k < A.nact; ++k) {  // the points that depend on this one
@@ -365,14 +361,18 @@ struct LinearVisitor {
                     const int y = __ldg(A.fidx + k * I.size_tot + n_t);
                     if (w == 0.f || y < 0 || (long long)y >= I.size_tot) continue;
                     const int ty = y / SIZE;
-                    if (ty == n_o) self = true;
-                    else push_tile<false>(S, I, ii, I.tile_base + ty, e);
+                    if (ty == n_o) continue;
+                    push_round(S, I.tile_base + ty, e);
+                    pushed = true;
                 }
             }
         }
         __syncwarp();
-        if (!settled && lane == 0) push_tile<false>(S, I, ii, t, e);
-        (void)self;
+        if (!settled && lane == 0) {
+            push_round(S, t, e);
+            pushed = true;
+        }
+        return pushed;
     }
 };
 

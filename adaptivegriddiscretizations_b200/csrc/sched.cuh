@@ -1,6 +1,6 @@
-// Device scheduler shared by the eikonal and the adjoint solvers: per-instance
-// epochs over tiles, one global queue of tiles, no grid-wide barrier.  See
-// eikonal.cu for the scheduling scheme.
+// Device schedulers shared by the eikonal and the adjoint solvers: per-instance
+// epochs over tiles, from one global queue of tiles without a grid-wide barrier
+// (sched_worker), or in rounds with one (rounds_worker).  See eikonal.cu.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -192,6 +192,9 @@ struct Ctrl {
     unsigned head, tail;       // global queue tickets (monotonic)
     int active;                // instances not finished
     unsigned err;
+    // Rounds (rounds_worker): arrivals at the end of the epochs of either parity
+    // (low half), and those of CTAs that pushed a tile (high half), a line each.
+    unsigned long long pad[14], round[2][16];
 };
 
 // Workspace: [Inst][InstState][tile_inst][lists][flags][score0][score1][queue][Ctrl][stats]
@@ -201,6 +204,13 @@ struct WsLayout {
     int nlists;  // epoch lists per instance (2, or kMaxLists with release epochs)
     unsigned qcap;
 };
+
+// Words of the tile bitmaps: three in tile order (queue), or two in owner order
+// (rounds: up to 31 padding bits per CTA).
+constexpr int kMaxRoundCtas = 148 * 4;
+static size_t bitmap_words(long long tiles) {
+    return std::max<size_t>(3 * ((tiles + 31) / 32), 2 * (tiles / 32 + 2 * kMaxRoundCtas));
+}
 
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr long long kMaxWarps = 148 * 64;  // resident warps of a launch, upper bound
@@ -249,7 +259,7 @@ static bool layout(const agd_instance *a, int n, WsLayout &L, Inst *out, bool st
     L.nlists = gated ? kMaxLists : 2;
     L.lists = off; off = align256(off + sizeof(int) * tiles * L.nlists);
     L.flags = off; off = align256(off + sizeof(unsigned) * tiles);
-    L.bits = off; off = align256(off + sizeof(unsigned) * 3 * ((tiles + 31) / 32));
+    L.bits = off; off = align256(off + sizeof(unsigned) * bitmap_words(tiles));
     L.score0 = off; off = align256(off + sizeof(unsigned) * tiles);
     L.score1 = off; off = align256(off + sizeof(unsigned) * tiles);
     L.queue = off; off = align256(off + sizeof(unsigned long long) * qcap);
@@ -300,8 +310,12 @@ struct Sched {
     // words each.
     unsigned *bits;
     unsigned nwords;
-    int bitmap;
+    int bitmap;  // kPushLists, kPushBits or kPushRounds
+    // Rounds: tile t belongs to CTA t % rctas, as bit t / rctas of its rwords
+    // words in the bitmap of its epoch's parity (rctas rwords words each).
+    unsigned rctas, rwords;
 };
+enum { kPushLists = 0, kPushBits = 1, kPushRounds = 2 };
 
 // Queue slot encoding: ticket (low 20 bits) << 44 | epoch << 30 | tile, empty =
 // all ones.  A consumer holding ticket h takes slot h % qcap only when it carries
@@ -339,6 +353,11 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -352,11 +371,16 @@ __device__ __forceinline__ int *list_of(const Sched &S, const Inst &I, int epoch
 // or, with release epochs, at its release epoch if that is later (at most
 // lmask epochs ahead).  The epoch a tile is pushed for never decreases, so the
 // epoch-stamped flag keeps one entry per tile and epoch.
-// BITMAP false: a visitor that never runs with bitmap pushes (its code stays
-// out of the visit).
-template <bool BITMAP = true>
+__device__ __forceinline__ void push_round(const Sched &S, int t, int e) {
+    const unsigned q = (unsigned)t / S.rctas, own = (unsigned)t - q * S.rctas;
+    atomicOr(S.bits + ((unsigned)(e + 1) & 1u) * S.rctas * S.rwords + own * S.rwords + (q >> 5), 1u << (q & 31u));
+}
 __device__ __forceinline__ void push_tile(const Sched &S, const Inst &I, int ii, int t, int e) {
-    if (BITMAP && S.bitmap) {  // a bit per tile and epoch: repeated pushes merge, and nothing waits for the result
+    if (S.bitmap == kPushRounds) {
+        push_round(S, t, e);
+        return;
+    }
+    if (S.bitmap == kPushBits) {  // a bit per tile and epoch: repeated pushes merge, and nothing waits for the result
         atomicOr(S.bits + (size_t)((unsigned)(e + 1) % 3u) * S.nwords + (t >> 5), 1u << (t & 31));
         return;
     }
@@ -393,44 +417,14 @@ __device__ __forceinline__ bool put_slot(const Sched &S, unsigned ticket, int ep
 }
 
 // Appends the n tile ids src[0..n), to be visited at epoch e, to the global queue;
-// warp-cooperative.  BULK: each lane handles kPubBatch entries at a time, their
-// list reads and slot checks issued together (one L2 round trip for 32 x
-// kPubBatch entries instead of one per 32), at the cost of the registers that
-// hold them; a slot still holding its previous lap's entry is waited for by
-// put_slot.
-constexpr int kPubBatch = 8;
-template <bool BULK>
+// warp-cooperative.
 static __device__ void enqueue_warp(const Sched &S, const int *src, int n, int e, int lane) {
     unsigned start = 0;
     if (lane == 0) start = atomicAdd(&S.ctrl->tail, (unsigned)n);
     start = __shfl_sync(kFull, start, 0);
     fence_acq_rel();  // release: the instance state and the tiles' values before the entries
-    if constexpr (BULK) {
-        bool ok = true;
-        for (int k0 = 0; k0 < n && ok; k0 += 32 * kPubBatch) {
-            int tile[kPubBatch];
-            unsigned long long prev[kPubBatch];
-#pragma unroll
-            for (int u = 0; u < kPubBatch; ++u) {
-                const int k = k0 + 32 * u + lane;
-                if (k < n) {
-                    tile[u] = __ldcg(src + k);
-                    prev[u] = ld_relaxed_u64(S.queue + (start + (unsigned)k) % S.qcap);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kPubBatch; ++u) {
-                const int k = k0 + 32 * u + lane;
-                if (k >= n || !ok) continue;
-                const unsigned ticket = start + (unsigned)k;
-                if (prev[u] == kSlotEmpty) st_relaxed_u64(S.queue + ticket % S.qcap, slot_word(ticket, e, (unsigned)tile[u]));
-                else ok = put_slot(S, ticket, e, (unsigned)tile[u]);
-            }
-        }
-    } else {
-        for (int k = lane; k < n; k += 32)
-            if (!put_slot(S, start + (unsigned)k, e, (unsigned)__ldcg(src + k))) break;
-    }
+    for (int k = lane; k < n; k += 32)
+        if (!put_slot(S, start + (unsigned)k, e, (unsigned)__ldcg(src + k))) break;
     __syncwarp();
 }
 
@@ -438,7 +432,6 @@ static __device__ void enqueue_warp(const Sched &S, const int *src, int n, int e
 // tile): publish the next list, or retire the instance.  The stop test is the
 // reference's: no tile left to update, or nitermax_o epochs run
 // (_solvers.py:94-120 with _StopCriterion.py:62-84, _solvers.py:53-57).
-template <bool BULK>
 static __device__ void close_epoch(const Sched &S, int ii, int e, int lane) {
     const Inst &I = S.inst[ii];
     InstState &st = S.ist[ii];
@@ -488,7 +481,7 @@ static __device__ void close_epoch(const Sched &S, int ii, int e, int lane) {
         __threadfence();
     }
     __syncwarp();
-    enqueue_warp<BULK>(S, list_of(S, I, en), n, en, lane);
+    enqueue_warp(S, list_of(S, I, en), n, en, lane);
 }
 
 
@@ -498,7 +491,6 @@ static __device__ void close_epoch(const Sched &S, int ii, int e, int lane) {
 // there.  Bitmap (e + 2) % 3, last read when epoch e - 1 closed, is cleared for
 // the pushes of epoch e + 1 before the entries go out; bitmap (e + 1) % 3 is
 // only read here, and cleared when epoch e + 2 closes.
-template <bool BULK>
 static __device__ void close_epoch_bitmap(const Sched &S, int ii, int e, int lane) {
     const Inst &I = S.inst[ii];
     InstState &st = S.ist[ii];
@@ -567,7 +559,7 @@ static __device__ void close_epoch_bitmap(const Sched &S, int ii, int e, int lan
         __threadfence();
     }
     __syncwarp();
-    enqueue_warp<BULK>(S, list, n, e + 1, lane);
+    enqueue_warp(S, list, n, e + 1, lane);
 }
 
 // Issues (lane 0) the copy of the 16 bytes that hold the queue slot of ticket h
@@ -628,12 +620,6 @@ __device__ __forceinline__ unsigned long long take_slot(const Sched &S, unsigned
 // Visitor provides: Args (by value), Smem (per warp), and
 //   static void visit(const Sched&, const Args&, int t, int ii, int e, int lane, Smem&).
 // Visitor::kMinCtas: resident 4-warp CTAs per SM that its register budget must allow.
-// Visitor::kBulkPublish: publish epochs with enqueue_warp<true> (more registers
-// in the worker loop, for visitors whose budget has them).
-// Visitor::kBatchScheduling: the worker may run launches of many instances with
-// the queue-slot prefetch, the ticket group taken ahead and bitmap pushes; a
-// visitor without it keeps the worker loop of one ticket ahead and list
-// pushes, and their registers (the linear visitor's budget has none to spare).
 constexpr int kSmemInst = 1024;  // instances whose tile bases a CTA keeps in shared memory
 
 // Decrement with release semantics (publishes this warp's writes); the warp
@@ -670,7 +656,7 @@ __global__ void __launch_bounds__(WPB * 32, Visitor::kMinCtas * 4 / WPB) sched_w
     // visit; a warp then holds up to 2 tgroup tickets (the exit sentinels of
     // close_epoch cover them).  Few instances keep one ticket ahead: a tile
     // held behind a busy warp lengthens their small epochs.
-    const bool ahead = Visitor::kBatchScheduling && S.tgroup > 1;
+    const bool ahead = S.tgroup > 1;
     unsigned ticket = 0, group = 0;
     int spare = 0;  // tickets of the group still ahead of `ticket`
     if (lane == 0) {
@@ -719,9 +705,152 @@ __global__ void __launch_bounds__(WPB * 32, Visitor::kMinCtas * 4 / WPB) sched_w
         lastone = __shfl_sync(kFull, lastone, 0);
         if (lastone) {
             fence_acq_rel();
-            if (Visitor::kBatchScheduling && S.bitmap) close_epoch_bitmap<Visitor::kBulkPublish>(S, ii, e, lane);
-            else close_epoch<Visitor::kBulkPublish>(S, ii, e, lane);
+            if (S.bitmap == kPushBits) close_epoch_bitmap(S, ii, e, lane);
+            else close_epoch(S, ii, e, lane);
         }
+    }
+}
+
+// ---------------------------------------------------------------- rounds ---
+// Launches of a few instances (fewer than kPairInstances, without release
+// epochs) run their epochs in rounds: one cooperative launch of resident CTAs,
+// every tile owned by one CTA, and a barrier of all the CTAs between epochs.
+// A push sets the tile's bit in its owner's words of the next epoch's bitmap
+// (fire and forget); a CTA starts an epoch by listing the bits of its own
+// words in shared memory, and its groups of warps visit the listed tiles.
+// Nothing is published tile by tile: in the queue above, one warp writes an
+// epoch's entries (120 tiles/us, 70 us of the 103 us that an epoch of an
+// Isotropic3 201^3 solve took), and every visit costs a ticket, a slot and a
+// counter round trip (39 us an epoch for a Riemann2 512^2 solve, of which the
+// visits of 400 tiles need a fraction).  Fixed owners also keep a tile's
+// read-only data in its SM's L1: the barrier polls with relaxed loads, which
+// leave L1 alone, and everything that other SMs write during the solve is read
+// through L2.  The instances of a launch share their epochs: an instance
+// without tiles in an epoch is finished (only its own visits push its tiles).
+// Many instances keep the queue, whose instances never wait for each other.
+//
+// Visitor provides: kRoundWarps (warps of a CTA), kRoundCtas (CTAs per
+// SM that the register budget must allow), kRoundG (warps of a group),
+// RoundSmem (per group), and
+//   static bool visit_round(const Sched&, const Args&, int t, int ii, int e, int tid, int group, RoundSmem&)
+// which returns whether the calling thread pushed a tile.
+constexpr int kRoundChunk = 64;  // words of own tiles listed at a time
+
+template <class Visitor>
+__global__ void __launch_bounds__(Visitor::kRoundWarps * 32, Visitor::kRoundCtas)
+    rounds_worker(const Sched S, const typename Visitor::Args VA) {
+    constexpr int G = Visitor::kRoundG, NW = Visitor::kRoundWarps, NG = NW / G;
+    static_assert(G == 1 || NG <= 15, "a named barrier per group");
+    extern __shared__ __align__(16) unsigned char round_smem[];
+    typename Visitor::RoundSmem *smem = reinterpret_cast<typename Visitor::RoundSmem *>(round_smem);
+    __shared__ int s_list[kRoundChunk * 32];
+    __shared__ int s_next[NG];
+    __shared__ int s_n, s_take, s_pushed, s_go;
+    __shared__ int s_base[kPairInstances], s_max[kPairInstances], s_flags[kPairInstances], s_last[kPairInstances];
+    __shared__ unsigned s_visits[kPairInstances];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int group = warp / G, gtid = tid - group * (32 * G);
+    for (int i = tid; i < S.ninst; i += NW * 32) {
+        s_base[i] = S.inst[i].tile_base;
+        s_max[i] = S.inst[i].a.nitermax_o;
+        s_flags[i] = S.inst[i].a.flags;
+        s_last[i] = 0;
+        s_visits[i] = 0u;
+    }
+    if (tid == 0) s_pushed = 0;
+    __syncthreads();
+    const unsigned half = S.rctas * S.rwords;
+    unsigned hi[2] = {0u, 0u};  // thread 0: the pushing arrivals seen, by parity
+    for (int e = 1;; ++e) {
+        unsigned *words = S.bits + (e & 1) * half + blockIdx.x * S.rwords;
+        for (unsigned c0 = 0; c0 < S.rwords; c0 += kRoundChunk) {
+            if (tid == 0) {
+                s_n = 0;
+                s_take = NG;
+            }
+            __syncthreads();
+            const unsigned c1 = min(S.rwords, c0 + kRoundChunk);
+            for (unsigned w = c0 + warp; w < c1; w += NW) {
+                const unsigned v = __ldcg(words + w);
+                if (v == 0u) continue;
+                const int t = (int)((w * 32 + lane) * S.rctas + blockIdx.x);
+                bool take = (v >> lane) & 1u;
+                if (take) {
+                    int ii = 0;
+                    for (int lo = 0, top = S.ninst - 1; lo < top; ii = lo) {
+                        const int mid = (lo + top + 1) >> 1;
+                        if (s_base[mid] <= t) lo = mid; else top = mid - 1;
+                    }
+                    // nitermax_o epochs at most (the first is always run); the global
+                    // iteration stops after an epoch without change
+                    if (e > 1 && e > s_max[ii]) take = false;
+                    if ((s_flags[ii] & AGD_FLAG_SOLVER_GLOBAL) && e > 1 && __ldcg(&S.ist[ii].changed) < e - 1) take = false;
+                    if (take) {
+                        s_last[ii] = e;
+                        atomicAdd(&s_visits[ii], 1u);
+                    }
+                }
+                const unsigned m = __ballot_sync(kFull, take);
+                int at = 0;
+                if (lane == 0) {
+                    words[w] = 0u;
+                    at = atomicAdd(&s_n, __popc(m));
+                }
+                at = __shfl_sync(kFull, at, 0);
+                if (take) s_list[at + __popc(m & ((1u << lane) - 1u))] = t;
+            }
+            __syncthreads();
+            const int n = s_n;
+            for (int i = group; i < n;) {
+                const int t = s_list[i];
+                int ii = 0;
+                for (int lo = 0, top = S.ninst - 1; lo < top; ii = lo) {
+                    const int mid = (lo + top + 1) >> 1;
+                    if (s_base[mid] <= t) lo = mid; else top = mid - 1;
+                }
+                if (gtid == 0) s_next[group] = atomicAdd(&s_take, 1);
+                if (Visitor::visit_round(S, VA, t, ii, e, gtid, group, smem[group])) s_pushed = 1;
+                if constexpr (G == 1) __syncwarp();
+                else asm volatile("barrier.cta.sync %0, %1;" ::"r"(group + 1), "n"(32 * G) : "memory");
+                i = s_next[group];
+                if constexpr (G > 1) asm volatile("barrier.cta.sync %0, %1;" ::"r"(group + 1), "n"(32 * G) : "memory");
+            }
+            __syncthreads();
+        }
+        if (tid == 0) {
+            // Everything this CTA wrote, then its arrival; nobody leaves the epoch
+            // before all have arrived.  A CTA is at most one epoch ahead of another,
+            // so the word of this parity is final once it counts every arrival.
+            unsigned long long *word = S.ctrl->round[e & 1];
+            const unsigned target = S.rctas * (unsigned)((e + 1) >> 1);
+            fence_acq_rel();
+            const unsigned long long one = 1ull | (s_pushed ? 1ull << 32 : 0ull);
+            asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(one) : "memory");
+            s_pushed = 0;
+            int go = -1;
+            const unsigned long long t0 = globaltimer();
+            for (unsigned it = 0; go < 0; ++it) {
+                const unsigned long long v = ld_relaxed_u64(word);
+                if ((unsigned)v >= target) {
+                    go = (unsigned)(v >> 32) != hi[e & 1];
+                    hi[e & 1] = (unsigned)(v >> 32);
+                } else if ((it & 7u) == 7u) {
+                    if (ld_relaxed_u32(&S.ctrl->err)) go = 0;
+                    else if (globaltimer() - t0 > S.timeout_ns) {
+                        atomicOr(&S.ctrl->err, (unsigned)AGD_STATUS_WATCHDOG);
+                        go = 0;
+                    }
+                }
+            }
+            s_go = go && e < kMaxEpochs;
+        }
+        __syncthreads();
+        if (!s_go) break;
+    }
+    for (int i = tid; i < S.ninst; i += NW * 32) {
+        if (s_last[i] == 0) continue;
+        atomicMax(&S.stats[i].niter_o, s_last[i]);
+        atomicAdd(reinterpret_cast<unsigned long long *>(&S.stats[i].tile_visits), (unsigned long long)s_visits[i]);
     }
 }
 
@@ -772,7 +901,9 @@ static __global__ void setup_tiles(Sched S, int total_tiles) {
             }
         }
     }
-    if (active) {
+    if (active && S.bitmap == kPushRounds) {
+        push_round(S, t, 0);
+    } else if (active) {
         S.flags[t] = 1u;
         const unsigned idx = atomicAdd(&S.ist[lo].cnt[1], 1u);
         list_of(S, I, 1)[idx] = t;
@@ -820,7 +951,11 @@ static __global__ void finish_stats(Sched S, agd_stats *out) {
     if (i >= S.ninst) return;
     agd_stats st = S.stats[i];
     st.status |= (int)S.ctrl->err;
-    if (!S.ist[i].done) st.status |= (int)AGD_STATUS_WATCHDOG;
+    if (S.bitmap == kPushRounds) {
+        if (st.niter_o > 0 && st.niter_o >= S.inst[i].a.nitermax_o) st.status |= (int)AGD_STATUS_NOT_CONVERGED;
+    } else if (!S.ist[i].done) {
+        st.status |= (int)AGD_STATUS_WATCHDOG;
+    }
     if (out) out[i] = st;
 }
 
@@ -848,6 +983,34 @@ static int launch_workers(const Sched &S, const typename Visitor::Args &VA, int 
     return AGD_STATUS_OK;
 }
 
+// The rounds' grid: resident CTAs (a cooperative launch), at most one per tile.
+template <class Visitor>
+static int rounds_ctas(int total_tiles, const agd_launch *cfg, int *ctas) {
+    auto kern = rounds_worker<Visitor>;
+    constexpr int smem = (int)sizeof(typename Visitor::RoundSmem) * (Visitor::kRoundWarps / Visitor::kRoundG);
+    int dev = 0, nsm = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return set_cuda_error("cudaGetDevice");
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return set_cuda_error("rounds shared memory");
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Visitor::kRoundWarps * 32, smem) != cudaSuccess)
+        return set_cuda_error("occupancy query");
+    if (per_sm < 1) return set_error(AGD_STATUS_UNSUPPORTED, "rounds kernel does not fit on an SM");
+    const int most = std::min(per_sm * nsm, kMaxRoundCtas);
+    int c = cfg && cfg->ctas > 0 ? cfg->ctas : total_tiles <= 16 * nsm ? nsm : most;
+    *ctas = std::max(1, std::min(std::min(c, most), total_tiles));
+    return AGD_STATUS_OK;
+}
+
+template <class Visitor>
+static int launch_rounds(const Sched &S, const typename Visitor::Args &VA, cudaStream_t st) {
+    constexpr int smem = (int)sizeof(typename Visitor::RoundSmem) * (Visitor::kRoundWarps / Visitor::kRoundG);
+    void *args[] = {const_cast<Sched *>(&S), const_cast<typename Visitor::Args *>(&VA)};
+    const cudaError_t err = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(rounds_worker<Visitor>),
+                                                        dim3(S.rctas), dim3(Visitor::kRoundWarps * 32), args, smem, st);
+    return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("rounds launch", err);
+}
+
 // Scheduler pointers inside a workspace laid out by layout().
 static Sched sched_at(const WsLayout &L, void *ws, int ninst) {
     char *w = static_cast<char *>(ws);
@@ -861,7 +1024,8 @@ static Sched sched_at(const WsLayout &L, void *ws, int ninst) {
     S.flags = reinterpret_cast<unsigned *>(w + L.flags);
     S.bits = reinterpret_cast<unsigned *>(w + L.bits);
     S.nwords = (unsigned)((L.total_tiles + 31) / 32);
-    S.bitmap = 0;
+    S.bitmap = kPushLists;
+    S.rctas = S.rwords = 0;
     S.score0 = reinterpret_cast<unsigned *>(w + L.score0);
     S.score1 = reinterpret_cast<unsigned *>(w + L.score1);
     S.queue = reinterpret_cast<unsigned long long *>(w + L.queue);
@@ -882,33 +1046,55 @@ static int run_sched(const WsLayout &L, void *ws, int n, const typename Visitor:
                      const agd_launch *cfg, cudaStream_t st) {
     Sched S = sched_at(L, ws, n);
     if (cfg && cfg->timeout_ns > 0) S.timeout_ns = (unsigned long long)cfg->timeout_ns;
-    // Bitmap pushes for launches of many instances: the pushes of a visit then
-    // wait for nothing, and an epoch is published in tile order.  A single
-    // instance keeps the lists, whose push order (the front's) propagates
-    // faster within an epoch when nothing else fills the GPU.
-    S.bitmap = (Visitor::kBatchScheduling && !Visitor::kBulkPublish && L.nlists == 2 && n >= kPairInstances) ? 1 : 0;
+    cudaError_t err;
     char *w = static_cast<char *>(ws);
-    cudaError_t err = cudaMemsetAsync(w + L.istate, 0, sizeof(InstState) * n, st);
-    if (err == cudaSuccess) err = cudaMemsetAsync(w + L.flags, 0, L.queue - L.flags, st);
-    if (err == cudaSuccess) err = cudaMemsetAsync(w + L.queue, 0xff, L.ctrl - L.queue, st);
-    // control block and stats; the stencil region after them is written in full by the stencil pass
-    if (err == cudaSuccess) err = cudaMemsetAsync(w + L.ctrl, 0, L.stencil - L.ctrl, st);
-    if (err != cudaSuccess) return set_cuda_error("workspace clear", err);
-    if ((err = Visitor::prepare(S, L, st)) != cudaSuccess) return set_cuda_error("prepare", err);
-    setup_tiles<<<(L.total_tiles + 255) / 256, 256, 0, st>>>(S, L.total_tiles);
-    if ((err = cudaGetLastError()) != cudaSuccess) return set_cuda_error("setup_tiles", err);
-    publish_first<<<(n + 127) / 128, 128, 0, st>>>(S);
-    publish_first_slots<<<(L.total_tiles + 255) / 256, 256, 0, st>>>(S, L.total_tiles);
-    if ((err = cudaGetLastError()) != cudaSuccess) return set_cuda_error("publish_first", err);
-    // 8-warp CTAs only where their static shared memory fits in 48 KB
-    constexpr bool kWide = (sizeof(typename Visitor::Smem) + 16) * 8 + sizeof(int) * kSmemInst <= 48 * 1024;
-    const int rc = (kWide && cfg && cfg->warps_per_cta == 8)
-                       ? launch_workers<Visitor, kWide ? 8 : 4>(S, VA, L.total_tiles, cfg, st)
-                       : launch_workers<Visitor, 4>(S, VA, L.total_tiles, cfg, st);
-    if (rc != AGD_STATUS_OK) return rc;
-    if ((err = Visitor::finalize(S, L, st)) != cudaSuccess) return set_cuda_error("finalize", err);
-    finish_stats<<<(n + 127) / 128, 128, 0, st>>>(S, stats);
-    if ((err = cudaGetLastError()) != cudaSuccess) return set_cuda_error("finish_stats", err);
+    if (Visitor::kQueueless || (n < kPairInstances && L.nlists == 2)) {
+        int ctas = 0;
+        const int rc = rounds_ctas<Visitor>(L.total_tiles, cfg, &ctas);
+        if (rc != AGD_STATUS_OK) return rc;
+        S.bitmap = kPushRounds;
+        S.rctas = (unsigned)ctas;
+        S.rwords = (unsigned)(((L.total_tiles + ctas - 1) / ctas + 31) / 32);
+        err = cudaMemsetAsync(w + L.istate, 0, sizeof(InstState) * n, st);
+        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.bits, 0, L.queue - L.bits, st);
+        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.ctrl, 0, L.stencil - L.ctrl, st);
+        if (err != cudaSuccess) return set_cuda_error("workspace clear", err);
+        if ((err = Visitor::prepare(S, L, st)) != cudaSuccess) return set_cuda_error("prepare", err);
+        setup_tiles<<<(L.total_tiles + 255) / 256, 256, 0, st>>>(S, L.total_tiles);
+        if ((err = cudaGetLastError()) != cudaSuccess) return set_cuda_error("setup_tiles", err);
+        const int rl = launch_rounds<Visitor>(S, VA, st);
+        if (rl != AGD_STATUS_OK) return rl;
+        if ((err = Visitor::finalize(S, L, st)) != cudaSuccess) return set_cuda_error("finalize", err);
+        finish_stats<<<(n + 127) / 128, 128, 0, st>>>(S, stats);
+        if ((err = cudaGetLastError()) != cudaSuccess) return set_cuda_error("finish_stats", err);
+        return AGD_STATUS_OK;
+    }
+    if constexpr (!Visitor::kQueueless) {  // the queue
+        // Bitmap pushes for launches of many instances: the pushes of a visit then
+        // wait for nothing, and an epoch is published in tile order.
+        S.bitmap = (L.nlists == 2 && n >= kPairInstances) ? kPushBits : kPushLists;
+        err = cudaMemsetAsync(w + L.istate, 0, sizeof(InstState) * n, st);
+        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.flags, 0, L.queue - L.flags, st);
+        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.queue, 0xff, L.ctrl - L.queue, st);
+        // control block and stats; the stencil region after them is written in full by the stencil pass
+        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.ctrl, 0, L.stencil - L.ctrl, st);
+        if (err != cudaSuccess) return set_cuda_error("workspace clear", err);
+        if ((err = Visitor::prepare(S, L, st)) != cudaSuccess) return set_cuda_error("prepare", err);
+        setup_tiles<<<(L.total_tiles + 255) / 256, 256, 0, st>>>(S, L.total_tiles);
+        if ((err = cudaGetLastError()) != cudaSuccess) return set_cuda_error("setup_tiles", err);
+        publish_first<<<(n + 127) / 128, 128, 0, st>>>(S);
+        publish_first_slots<<<(L.total_tiles + 255) / 256, 256, 0, st>>>(S, L.total_tiles);
+        if ((err = cudaGetLastError()) != cudaSuccess) return set_cuda_error("publish_first", err);
+        // 8-warp CTAs only where their static shared memory fits in 48 KB
+        constexpr bool kWide = (sizeof(typename Visitor::Smem) + 16) * 8 + sizeof(int) * kSmemInst <= 48 * 1024;
+        const int rc = (kWide && cfg && cfg->warps_per_cta == 8)
+                           ? launch_workers<Visitor, kWide ? 8 : 4>(S, VA, L.total_tiles, cfg, st)
+                           : launch_workers<Visitor, 4>(S, VA, L.total_tiles, cfg, st);
+        if (rc != AGD_STATUS_OK) return rc;
+        if ((err = Visitor::finalize(S, L, st)) != cudaSuccess) return set_cuda_error("finalize", err);
+        finish_stats<<<(n + 127) / 128, 128, 0, st>>>(S, stats);
+        if ((err = cudaGetLastError()) != cudaSuccess) return set_cuda_error("finish_stats", err);
+    }
     return AGD_STATUS_OK;
 }
 
