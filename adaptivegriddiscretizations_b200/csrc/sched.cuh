@@ -733,8 +733,33 @@ __global__ void __launch_bounds__(WPB * 32, Visitor::kMinCtas * 4 / WPB) sched_w
 // SM that the register budget must allow), kRoundG (warps of a group),
 // RoundSmem (per group), and
 //   static bool visit_round(const Sched&, const Args&, int t, int ii, int e, int tid, int group, RoundSmem&)
-// which returns whether the calling thread pushed a tile.
+// which returns whether the calling thread pushed a tile, and
+//   static bool due(const Args&, int t, int e)
+// (kOrdered true): a tile pushed before it is due waits.
 constexpr int kRoundChunk = 64;  // words of own tiles listed at a time
+
+// Barrier of a group of G warps, and its vote.  Groups of several warps use a
+// named barrier (1 + the group's index in the CTA: at most 15 such groups).
+template <int G>
+__device__ __forceinline__ void group_sync(int group) {
+    if constexpr (G == 1) __syncwarp();
+    else asm volatile("barrier.cta.sync %0, %1;" ::"r"(group + 1), "n"(32 * G) : "memory");
+}
+template <int G>
+__device__ __forceinline__ bool group_any(int group, bool x) {
+    if constexpr (G == 1) {
+        return __any_sync(kFull, x);
+    } else {
+        int r;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\t"
+            "barrier.cta.red.or.pred q, %2, %3, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+            : "=r"(r)
+            : "r"((int)x), "r"(group + 1), "n"(32 * G)
+            : "memory");
+        return r != 0;
+    }
+}
 
 template <class Visitor>
 __global__ void __launch_bounds__(Visitor::kRoundWarps * 32, Visitor::kRoundCtas)
@@ -775,6 +800,14 @@ __global__ void __launch_bounds__(Visitor::kRoundWarps * 32, Visitor::kRoundCtas
                 if (v == 0u) continue;
                 const int t = (int)((w * 32 + lane) * S.rctas + blockIdx.x);
                 bool take = (v >> lane) & 1u;
+                if constexpr (Visitor::kOrdered) {
+                    const unsigned wait = __ballot_sync(kFull, take && !Visitor::due(VA, t, e));
+                    if (wait && lane == 0) {
+                        atomicOr(S.bits + ((e + 1) & 1) * half + blockIdx.x * S.rwords + w, wait);
+                        s_pushed = 1;
+                    }
+                    take = take && !((wait >> lane) & 1u);
+                }
                 if (take) {
                     int ii = 0;
                     for (int lo = 0, top = S.ninst - 1; lo < top; ii = lo) {
@@ -810,10 +843,9 @@ __global__ void __launch_bounds__(Visitor::kRoundWarps * 32, Visitor::kRoundCtas
                 }
                 if (gtid == 0) s_next[group] = atomicAdd(&s_take, 1);
                 if (Visitor::visit_round(S, VA, t, ii, e, gtid, group, smem[group])) s_pushed = 1;
-                if constexpr (G == 1) __syncwarp();
-                else asm volatile("barrier.cta.sync %0, %1;" ::"r"(group + 1), "n"(32 * G) : "memory");
+                group_sync<G>(group);
                 i = s_next[group];
-                if constexpr (G > 1) asm volatile("barrier.cta.sync %0, %1;" ::"r"(group + 1), "n"(32 * G) : "memory");
+                group_sync<G>(group);
             }
             __syncthreads();
         }

@@ -270,26 +270,8 @@ struct Visit {
             return tid + NT * p;
         }
     }
-    // Barrier of the group, and its vote.  Groups of several warps use a named
-    // barrier (1 + the group's index in the CTA: at most 15 such groups).
-    __device__ __forceinline__ static void gsync(int group) {
-        if constexpr (G == 1) __syncwarp();
-        else asm volatile("barrier.cta.sync %0, %1;" ::"r"(group + 1), "n"(NT) : "memory");
-    }
-    __device__ __forceinline__ static bool gany(int group, bool x) {
-        if constexpr (G == 1) {
-            return __any_sync(kFull, x);
-        } else {
-            int r;
-            asm volatile(
-                "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\t"
-                "barrier.cta.red.or.pred q, %2, %3, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
-                : "=r"(r)
-                : "r"((int)x), "r"(group + 1), "n"(NT)
-                : "memory");
-            return r != 0;
-        }
-    }
+    __device__ __forceinline__ static void gsync(int group) { group_sync<G>(group); }
+    __device__ __forceinline__ static bool gany(int group, bool x) { return group_any<G>(group, x); }
     static constexpr int kSmemFloats = kSlots ? TL::SIZE * (1 + (ORD2 ? 2 : 1) * NTOT) : 2 * TL::SIZE;
     __device__ __forceinline__ static float neighbour(float x, const float *us) {
         const int b = __float_as_int(x);
@@ -939,6 +921,7 @@ struct EikonalVisitor {
     struct RoundSmem {
         float u[smem_floats<VMASK, kRoundG>()];
     };
+    static constexpr bool kOrdered = false;
     __device__ __forceinline__ static bool visit_round(const Sched &S, const Args &, int t, int ii, int e, int tid,
                                                        int group, RoundSmem &sm) {
         return dispatch<VMASK, kRoundG>(S, t, ii, e, tid, group, sm.u);
