@@ -287,18 +287,18 @@ class UNet:
     def step(self, lr, beta1=0.9, beta2=0.999, eps=1e-8):
         """One Adam step on every weight; clears the gradients."""
         self.t += 1
-        L = _lib.lib()
-        s = _lib.stream_ptr()
-        for layer in self.layers():
-            _lib.check(L.agd_ws_adam(_p(layer.w), _p(layer.dw), _p(layer.mw), _p(layer.vw), layer.w.numel(),
-                                     lr, beta1, beta2, eps, self.t, _p(layer.wb), s), "adam")
-            _lib.check(L.agd_ws_adam(_p(layer.b), _p(layer.db), _p(layer.mb), _p(layer.vb), layer.b.numel(),
-                                     lr, beta1, beta2, eps, self.t, None, s), "adam")
-            layer.flip()
-        _lib.check(L.agd_ws_adam(_p(self.hw), _p(self.dhw), _p(self.mhw), _p(self.vhw), self.hw.numel(), lr,
-                                 beta1, beta2, eps, self.t, None, s), "adam")
-        _lib.check(L.agd_ws_adam(_p(self.hb), _p(self.dhb), _p(self.mhb), _p(self.vhb), 1, lr, beta1, beta2, eps,
-                                 self.t, None, s), "adam")
+        tensors = [(layer.w, layer.dw, layer.mw, layer.vw, layer.wb, layer.wt, layer.cin, layer.cout)
+                   for layer in self.layers()]
+        tensors += [(layer.b, layer.db, layer.mb, layer.vb, None, None, 0, 0) for layer in self.layers()]
+        tensors += [(self.hw, self.dhw, self.mhw, self.vhw, None, None, 0, 0),
+                    (self.hb, self.dhb, self.mhb, self.vhb, None, None, 0, 0)]
+        arr = (_lib.AgdAdamTensor * len(tensors))()
+        for a, (w, g, m, v, wb, wt, cin, cout) in zip(arr, tensors):
+            a.w, a.g, a.m, a.v, a.n = w.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), w.numel()
+            if wb is not None:
+                a.wb, a.wt, a.cin, a.cout = wb.data_ptr(), wt.data_ptr(), cin, cout
+        _lib.check(_lib.lib().agd_ws_adam_list(arr, len(tensors), lr, beta1, beta2, eps, self.t, _lib.stream_ptr()),
+                   "adam")
 
     def zero_grad(self):
         for layer in self.layers():

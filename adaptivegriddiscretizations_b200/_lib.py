@@ -74,6 +74,12 @@ class AgdConv(ctypes.Structure):
                 ("cout", ctypes.c_int)]
 
 
+class AgdAdamTensor(ctypes.Structure):
+    _fields_ = [("w", ctypes.c_void_p), ("g", ctypes.c_void_p), ("m", ctypes.c_void_p), ("v", ctypes.c_void_p),
+                ("wb", ctypes.c_void_p), ("wt", ctypes.c_void_p), ("n", ctypes.c_int64), ("cin", ctypes.c_int),
+                ("cout", ctypes.c_int)]
+
+
 class AgdWsTerm(ctypes.Structure):
     _fields_ = [("data", ctypes.c_void_p), ("mode", ctypes.c_int), ("channels", ctypes.c_int),
                 ("offset", ctypes.c_int)]
@@ -124,6 +130,8 @@ SIGNATURES = {
     "agd_ws_bias_grad": (_I, [_P, ctypes.c_longlong, _I, _P, _P]),
     "agd_ws_head_forward": (_I, [_P, ctypes.c_longlong, _P, _P, _P, _P]),
     "agd_ws_head_loss_backward": (_I, [_P, ctypes.c_longlong, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _P, _P]),
+    "agd_ws_adam_list": (_I, [ctypes.POINTER(AgdAdamTensor), _I, ctypes.c_float, ctypes.c_float, ctypes.c_float,
+                              ctypes.c_float, _I, _P]),
     "agd_ws_adam": (_I, [_P, _P, _P, _P, ctypes.c_longlong, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                          ctypes.c_float, _I, _P, _P]),
     "agd_ws_release": (_I, [_P, _I, _I, _I, ctypes.c_float, _I, _P, _P]),

@@ -124,6 +124,19 @@ int agd_ws_head_loss_backward(const void *y, long long M, const float *w, const 
 int agd_ws_adam(float *w, float *g, float *m, float *v, long long n, float lr, float beta1, float beta2, float eps,
                 int t, void *wb, agd_stream_t stream);
 
+/* agd_ws_adam over a list of tensors (host array), all at step t, in one launch.
+ * wb as in agd_ws_adam; wt (with wb, the (cout, agd_conv_kpad(cin)) weights of a
+ * convolution) may be the flipped copy of agd_conv_weight_flip, whose padding
+ * columns are not written, or NULL. */
+typedef struct agd_ws_adam_tensor {
+    float *w, *g, *m, *v;
+    void *wb, *wt;
+    int64_t n;
+    int cin, cout;
+} agd_ws_adam_tensor;
+int agd_ws_adam_list(const agd_ws_adam_tensor *list, int count, float lr, float beta1, float beta2, float eps, int t,
+                     agd_stream_t stream);
+
 /* Release epochs of 8x8 tiles from block predictions of the arrival time
  * (n, Hb, Wb) fp32 (one value per 4x4 block): release = max(1, 1 +
  * floor(epochs tmin / tmax) - lag), tmin the tile's smallest prediction, tmax
