@@ -1181,38 +1181,39 @@ class Interface:
             max_chunks = int(np.ceil(float(max_len) / typical_len))
         tips = self.tips
         ntips = int(tips.shape[0])
-        seed_mask = torch.zeros(self.shape, dtype=torch.uint8, device="cuda")
-        seed_mask[tuple(torch.as_tensor(self.seedIndices.T, device="cuda").long())] = 1
+        npasses, cut = int(np.ceil(eucl_bound)), int(5 * eucl_bound)
         eucl = torch.empty(self.shape, dtype=torch.uint8, device="cuda")
-        tmp = torch.empty_like(eucl)
-        _lib.check(L.agd_eucl_map(self.ndim, self.c_shape, _lib.ptr(seed_mask), int(np.ceil(eucl_bound)),
-                                  int(5 * eucl_bound), _lib.ptr(eucl), _lib.ptr(tmp), self.stream), "eucl")
-        start = torch.as_tensor(self.hfmIn.corners[0] + 0.5 * self.hfmIn.gridScales, device="cuda")
-        hh = torch.as_tensor(self.h, device="cuda")
+        # a few seeds: the boxes around them; many, or a wide bound: passes over the grid
+        nbox = len(self.seedIndices) * (2 * npasses + 1) ** self.ndim
+        if 0 <= npasses <= 255 and nbox <= 1 << 15:
+            _lib.check(L.agd_eucl_map_seeds(self.ndim, self.c_shape, _lib.ptr(self.seed_idx_t), len(self.seedIndices),
+                                            npasses, cut, _lib.ptr(eucl), self.stream), "eucl")
+        else:
+            seed_mask = torch.zeros(self.shape, dtype=torch.uint8, device="cuda")
+            seed_mask[tuple(torch.as_tensor(self.seedIndices.T, device="cuda").long())] = 1
+            tmp = torch.empty_like(eucl)
+            _lib.check(L.agd_eucl_map(self.ndim, self.c_shape, _lib.ptr(seed_mask), npasses, cut, _lib.ptr(eucl),
+                                      _lib.ptr(tmp), self.stream), "eucl")
+        origin = np.asarray(self.hfmIn.corners[0] + 0.5 * self.hfmIn.gridScales)
+        start, hh = torch.as_tensor(np.stack([origin, self.h.astype(origin.dtype)]), device="cuda")  # one upload
         tips_c = ((tips.float() - start) / hh).contiguous()
         cap = max_chunks * (typical_len - 1) + 1
         paths = torch.empty((ntips, cap, self.ndim), dtype=torch.float32, device="cuda")
-        lengths = torch.empty(ntips, dtype=torch.int32, device="cuda")
-        stops = torch.empty(ntips, dtype=torch.int8, device="cuda")
+        ends = torch.empty(5 * ntips, dtype=torch.uint8, device="cuda")  # lengths (int32), then stops: one readback
         inst = self.instance()
         _lib.check(L.agd_geodesics(ctypes.byref(inst), _lib.ptr(self.flow_vector), _lib.ptr(self.flow_weightsum),
                                    _lib.ptr(eucl), _lib.ptr(tips_c), ntips, ctypes.c_float(step),
                                    ctypes.c_float(causality), typical_len, max_chunks, eucl_delay, nymin_delay,
-                                   pastseed_delay, _lib.ptr(paths), cap, _lib.ptr(lengths), _lib.ptr(stops), self.stream),
-                   "geodesics")
-        lens = lengths.cpu().numpy()
-        codes = stops.cpu().numpy()
+                                   pastseed_delay, _lib.ptr(paths), cap, _lib.ptr(ends),
+                                   ctypes.c_void_p(ends.data_ptr() + 4 * ntips), self.stream), "geodesics")
+        ends = ends.cpu().numpy()
+        lens, codes = ends[: 4 * ntips].view(np.int32).tolist(), ends[4 * ntips:].view(np.int8).tolist()
         # all paths to physical coordinates at once; each geodesic is a (ndim, len)
         # view, transposed like the reference's PointFromIndex(geo).T
-        maxlen = int(lens.max()) if ntips else 0
-        phys = paths[:, :maxlen] * hh + start
-        geos = [phys[i, : int(lens[i])].T for i in range(ntips)]
-        crit = []
-        for i in range(ntips):
-            if codes[i] == 0:
-                crit.append("Stopping criterion")
-            else:
-                crit.append(GEODESIC_CODES[int(codes[i])])
+        maxlen = max(lens) if ntips else 0
+        phys = (paths[:, :maxlen] * hh + start).transpose(1, 2).unbind(0)
+        geos = [g if n == maxlen else g.narrow(1, 0, n) for g, n in zip(phys, lens)]
+        crit = ["Stopping criterion" if c == 0 else GEODESIC_CODES[c] for c in codes]
         if any(c == "Stopping criterion" for c in crit):
             self.Warn("Geodesic solver failed to converge, or geodesic has too many points"
                       " (in latter case, try setting 'geodesic_max_length':np.inf)")

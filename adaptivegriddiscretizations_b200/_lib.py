@@ -112,6 +112,7 @@ SIGNATURES = {
     "agd_eucl_map": (_I, [_I, _P, _P, _I, _I, _P, _P, _P]),
     "agd_geodesics": (_I, [_P, _P, _P, _P, _P, _I, ctypes.c_float, ctypes.c_float, _I, _I, _I, _I, _I, _P, _I,
                            _P, _P, _P]),
+    "agd_eucl_map_seeds": (_I, [_I, _P, _P, _I, _I, _I, _P, _P]),
     "agd_reverse_workspace_bytes": (ctypes.c_size_t, [_P]),
     "agd_reverse": (_I, [_P, _P, _P, _P, _P, _P, ctypes.c_float, ctypes.c_float, _P, ctypes.c_size_t, _P, _P,
                          _P]),

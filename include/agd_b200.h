@@ -353,6 +353,12 @@ int agd_geodesics(const agd_instance *inst, const float *flow_vector, const floa
 /* Workspace for agd_reverse. */
 size_t agd_reverse_workspace_bytes(const agd_instance *inst);
 
+/* agd_eucl_map of a few seeds given by their grid indices ((nseeds, ndim) int32,
+ * those outside the grid ignored): the same map, by the costs of the shortest
+ * paths in a box around each seed instead of passes over the grid. */
+int agd_eucl_map_seeds(int ndim, const int *shape, const int32_t *seed_index, int nseeds, int npasses, int cut,
+                       uint8_t *eucl, agd_stream_t stream);
+
 /* Reverse-mode sensitivity: solves diag*lam - W^T lam = sens on the tiles, where
  * W holds the upwind flow weights (flow_weights/flow_indices of agd_flow) and
  * diag = flow_weightsum (1 where it vanishes).  sens, lam: tile layout.
