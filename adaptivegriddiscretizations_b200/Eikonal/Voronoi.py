@@ -49,14 +49,16 @@ def _offset_dtype(offset_t):
     return t
 
 
-def _decompose(m_flat, ndim, offset_t):
-    """Kernel call on (symdim, n) float32 CUDA planes; returns weights, offsets."""
-    sd, n = m_flat.shape
-    w = torch.empty((sd, n), dtype=torch.float32, device=m_flat.device)
-    e = torch.empty((ndim, sd, n), dtype=offset_t, device=m_flat.device)
+def _decompose(m, ndim, offset_t, full=False):
+    """Kernel call on (symdim, n) float32 CUDA planes, or with full on matrices
+    (ndim, ndim, n); returns weights, offsets."""
+    sd, n = ndim * (ndim + 1) // 2, m.shape[-1]
+    w = torch.empty((sd, n), dtype=torch.float32, device=m.device)
+    e = torch.empty((ndim, sd, n), dtype=offset_t, device=m.device)
     L = _lib.lib()
-    _lib.check(L.agd_voronoi_decomposition(ndim, _lib.ptr(m_flat), n, _lib.ptr(w), _lib.ptr(e),
-                                           _OFFSET_BYTES[offset_t], _lib.stream_ptr()), "voronoi_decomposition")
+    fn = L.agd_voronoi_matrices if full else L.agd_voronoi_decomposition
+    _lib.check(fn(ndim, _lib.ptr(m), n, _lib.ptr(w), _lib.ptr(e), _OFFSET_BYTES[offset_t], _lib.stream_ptr()),
+               "voronoi_decomposition")
     return w, e
 
 
@@ -106,17 +108,23 @@ def VoronoiDecomposition(arr, mode=None, steps="Both", offset_t=torch.int32, fla
     host = not isinstance(arr, torch.Tensor)
     t = torch.as_tensor(np.asarray(arr) if host else arr)
     t = t.to(device="cuda", dtype=torch.float32) if t.dtype != torch.float32 or not t.is_cuda else t
-    m_flat = t if flattened else flatten_symmetric_matrix(t)
-    sd = m_flat.shape[0]
-    ndim = {1: 1, 3: 2, 6: 3}.get(sd)
-    if ndim is None or (not flattened and t.shape[1] != ndim):
-        raise ValueError(f"Voronoi decomposition not implemented in dimension {int(np.sqrt(2 * sd))} "
-                         "(dimensions 1 to 3 here)")
-    shape = tuple(m_flat.shape[1:])
-    flat2 = m_flat.reshape(sd, -1)
-    w, e = _decompose(flat2.detach().contiguous(), ndim, offset_t)
-    if flat2.requires_grad:
-        w = _Weights.apply(flat2, w, e)
+    if not flattened and t.dim() >= 2 and t.shape[0] == t.shape[1] <= 3 and not t.requires_grad:
+        # matrices without a gradient: the kernel reads their lower triangles in place
+        ndim = t.shape[0]
+        sd, shape = ndim * (ndim + 1) // 2, tuple(t.shape[2:])
+        w, e = _decompose(t.reshape(ndim, ndim, -1).contiguous(), ndim, offset_t, full=True)
+    else:
+        m_flat = t if flattened else flatten_symmetric_matrix(t)
+        sd = m_flat.shape[0]
+        ndim = {1: 1, 3: 2, 6: 3}.get(sd)
+        if ndim is None or (not flattened and t.shape[1] != ndim):
+            raise ValueError(f"Voronoi decomposition not implemented in dimension {int(np.sqrt(2 * sd))} "
+                             "(dimensions 1 to 3 here)")
+        shape = tuple(m_flat.shape[1:])
+        flat2 = m_flat.reshape(sd, -1)
+        w, e = _decompose(flat2.detach().contiguous(), ndim, offset_t)
+        if flat2.requires_grad:
+            w = _Weights.apply(flat2, w, e)
     w = w.reshape((sd,) + shape)
     e = e.reshape((ndim, sd) + shape)
     if mode == "gpu_transfer":

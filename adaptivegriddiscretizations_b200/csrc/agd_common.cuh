@@ -136,6 +136,111 @@ done:
     w[5] = fmaxf(0.f, -scal_vmv<3>(b2, m, b3)); cross3(b0, b1, e[5]);
 }
 
+// The same reductions with the superbase in float: its entries and the products
+// of pairs of them are small integers, exact in float as long as no entry
+// reaches 2048 in magnitude, so the result is the same bit for bit without an
+// integer multiply and conversion per term.  Larger superbases are done
+// again in integers.  (Selling's reduction of 1.3 M 3x3 matrices: 59 -> 45 us.)
+template <int D>
+__device__ __forceinline__ float scal_vmv_f(const float *x, const float *m, const float *y) {
+    float r = 0.f;
+    int k = 0;
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j, ++k) r += (i == j ? x[i] * y[i] : x[i] * y[j] + x[j] * y[i]) * m[k];
+    return r;
+}
+static __device__ __noinline__ void selling2_again(const float *m, float *w, int (*e)[3]) { selling2(m, w, e); }
+static __device__ __noinline__ void selling3_again(const float *m, float *w, int (*e)[3]) { selling3(m, w, e); }
+
+__device__ __forceinline__ void selling2_fast(const float *m, float *w, int (*e)[3]) {
+    float b0[2] = {1, 0}, b1[2] = {0, 1}, b2[2] = {-1, -1}, big = 1.f;
+    int iter = 0, red = 0;
+#define AGD_SELL2_STEP(BI, BJ, BK)                                   \
+    if (iter >= 100 || red >= 3) goto done;                          \
+    if (scal_vmv_f<2>(BI, m, BJ) > 0.f) {                            \
+        BK[0] = BI[0] - BJ[0]; BK[1] = BI[1] - BJ[1];                 \
+        BI[0] = -BI[0]; BI[1] = -BI[1];                              \
+        big = fmaxf(big, fmaxf(fabsf(BK[0]), fabsf(BK[1])));         \
+        red = 0;                                                     \
+    }                                                                \
+    ++iter; ++red;
+    while (true) {
+        AGD_SELL2_STEP(b0, b1, b2)
+        AGD_SELL2_STEP(b1, b2, b0)
+        AGD_SELL2_STEP(b2, b0, b1)
+    }
+#undef AGD_SELL2_STEP
+done:
+    if (!(big < 2048.f)) {
+        float mm[3] = {m[0], m[1], m[2]}, ww[3];
+        int ee[3][3];
+        selling2_again(mm, ww, ee);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            w[k] = ww[k];
+            e[k][0] = ee[k][0];
+            e[k][1] = ee[k][1];
+        }
+        return;
+    }
+    w[0] = fmaxf(0.f, -scal_vmv_f<2>(b0, m, b1)); e[0][0] = -(int)b2[1]; e[0][1] = (int)b2[0];
+    w[1] = fmaxf(0.f, -scal_vmv_f<2>(b1, m, b2)); e[1][0] = -(int)b0[1]; e[1][1] = (int)b0[0];
+    w[2] = fmaxf(0.f, -scal_vmv_f<2>(b2, m, b0)); e[2][0] = -(int)b1[1]; e[2][1] = (int)b1[0];
+}
+
+__device__ __forceinline__ void cross3f(const float *a, const float *b, int *o) {
+    o[0] = (int)(a[1] * b[2] - a[2] * b[1]);
+    o[1] = (int)(a[2] * b[0] - a[0] * b[2]);
+    o[2] = (int)(a[0] * b[1] - a[1] * b[0]);
+}
+
+__device__ __forceinline__ void selling3_fast(const float *m, float *w, int (*e)[3]) {
+    float b0[3] = {1, 0, 0}, b1[3] = {0, 1, 0}, b2[3] = {0, 0, 1}, b3[3] = {-1, -1, -1}, big = 1.f;
+    int iter = 0, red = 0;
+#define AGD_SELL3_STEP(BI, BJ, BK, BL)                               \
+    if (iter >= 100 || red >= 6) goto done;                          \
+    if (scal_vmv_f<3>(BI, m, BJ) > 0.f) {                            \
+        _Pragma("unroll") for (int c = 0; c < 3; ++c) {              \
+            BK[c] += BI[c]; BL[c] += BI[c]; BI[c] = -BI[c];          \
+            big = fmaxf(big, fmaxf(fabsf(BK[c]), fabsf(BL[c])));     \
+        }                                                            \
+        red = 0;                                                     \
+    }                                                                \
+    ++iter; ++red;
+    while (true) {
+        AGD_SELL3_STEP(b0, b1, b2, b3)
+        AGD_SELL3_STEP(b0, b2, b1, b3)
+        AGD_SELL3_STEP(b0, b3, b1, b2)
+        AGD_SELL3_STEP(b1, b2, b0, b3)
+        AGD_SELL3_STEP(b1, b3, b0, b2)
+        AGD_SELL3_STEP(b2, b3, b0, b1)
+    }
+#undef AGD_SELL3_STEP
+done:
+    if (!(big < 2048.f)) {
+        float mm[6], ww[6];
+        int ee[6][3];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) mm[k] = m[k];
+        selling3_again(mm, ww, ee);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            w[k] = ww[k];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) e[k][c] = ee[k][c];
+        }
+        return;
+    }
+    w[0] = fmaxf(0.f, -scal_vmv_f<3>(b0, m, b1)); cross3f(b2, b3, e[0]);
+    w[1] = fmaxf(0.f, -scal_vmv_f<3>(b0, m, b2)); cross3f(b1, b3, e[1]);
+    w[2] = fmaxf(0.f, -scal_vmv_f<3>(b0, m, b3)); cross3f(b1, b2, e[2]);
+    w[3] = fmaxf(0.f, -scal_vmv_f<3>(b1, m, b2)); cross3f(b0, b3, e[3]);
+    w[4] = fmaxf(0.f, -scal_vmv_f<3>(b1, m, b3)); cross3f(b0, b2, e[4]);
+    w[5] = fmaxf(0.f, -scal_vmv_f<3>(b2, m, b3)); cross3f(b0, b1, e[5]);
+}
+
 // ------------------------------------------------------ eikonal operator ---
 // Sorting network on (value, weight) pairs, ascending values.  A comparator
 // keeps its pair only when strictly ordered, which is the tie rule of the

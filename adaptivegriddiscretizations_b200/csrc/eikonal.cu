@@ -276,7 +276,15 @@ __global__ void flow_kernel(Inst I, float *fvec, float *fwsum, float *fw, int *f
         const bool seed = (__ldg(A.seedbits + (n_t >> 3)) >> (n_t & 7)) & 1;
         float w[NACT], fwk[NACT];
         int ev[NACT][3], side[NACT];
-        V::stencil(I, n_t, w, ev);
+        if constexpr (V::kSelling) {
+            float m[V::SD];
+#pragma unroll
+            for (int c = 0; c < V::SD; ++c) m[c] = __ldg(A.geom + (size_t)c * I.size_tot + n_t);
+            if (D == 2) selling2_fast(m, w, ev);
+            else selling3_fast(m, w, ev);
+        } else {
+            V::stencil(I, n_t, w, ev);
+        }
         unsigned hide[NACT];  // neighbours hidden by a wall (Riemann offsets; see Visit::stencil_decode)
         const int wd0 = (V::kSelling && A.wall_dist && in) ? (int)__ldg(A.wall_dist + n_t) : 255;
 #pragma unroll
@@ -769,10 +777,11 @@ __global__ void wall_dist_batch_kernel(Geo g, int nb, const uint8_t *dist, uint8
 
 // Selling's decomposition of n packed symmetric matrices in the planar layouts
 // of the reference's VoronoiDecomposition kernel (Kernel_VoronoiDecomposition.h:45-69):
-// m[c * n + p] (lower triangle, row major), weights[r * n + p],
+// m[c * n + p] (lower triangle, row major; FULL: the whole matrices, m[(i D + j)
+// n + p], of which the lower triangle is read), weights[r * n + p],
 // offsets[(i * SD + r) * n + p] for coordinate i of offset r.  Dimension 1: the
 // weight is the matrix, the offset 1.  One thread per matrix, grid stride.
-template <int D, class OffT>
+template <int D, class OffT, bool FULL>
 __global__ void voronoi_kernel(const float *__restrict__ m, long long n, float *__restrict__ w,
                                OffT *__restrict__ e) {
     constexpr int SD = D * (D + 1) / 2;
@@ -780,32 +789,32 @@ __global__ void voronoi_kernel(const float *__restrict__ m, long long n, float *
         float mm[SD], ww[SD];
         int ee[SD][3];
 #pragma unroll
-        for (int c = 0; c < SD; ++c) mm[c] = __ldg(m + c * n + p);
+            for (int j = 0; j <= i; ++j, ++c) mm[c] = __ldg(m + (FULL ? i * D + j : c) * n + p);
         if constexpr (D == 1) {
             ww[0] = mm[0];
             ee[0][0] = 1;
         } else if constexpr (D == 2) {
-            selling2(mm, ww, ee);
+            selling2_fast(mm, ww, ee);
         } else {
-            selling3(mm, ww, ee);
+            selling3_fast(mm, ww, ee);
         }
 #pragma unroll
         for (int r = 0; r < SD; ++r) {
-            w[r * n + p] = ww[r];
+            __stcs(w + r * n + p, ww[r]);
 #pragma unroll
-            for (int i = 0; i < D; ++i) e[(i * SD + r) * n + p] = (OffT)ee[r][i];
+            for (int i = 0; i < D; ++i) __stcs(e + (i * SD + r) * n + p, (OffT)ee[r][i]);
         }
     }
 }
 
-template <int D>
+template <int D, bool FULL>
 static void launch_voronoi(const float *m, long long n, float *w, void *e, int offset_bytes, cudaStream_t st) {
-    const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 32);
+    const unsigned blocks = (unsigned)std::min<long long>((n + 127) / 128, 148LL * 64);
     switch (offset_bytes) {
-        case 1: voronoi_kernel<D, int8_t><<<blocks, 256, 0, st>>>(m, n, w, static_cast<int8_t *>(e)); break;
-        case 2: voronoi_kernel<D, int16_t><<<blocks, 256, 0, st>>>(m, n, w, static_cast<int16_t *>(e)); break;
-        case 4: voronoi_kernel<D, int32_t><<<blocks, 256, 0, st>>>(m, n, w, static_cast<int32_t *>(e)); break;
-        default: voronoi_kernel<D, int64_t><<<blocks, 256, 0, st>>>(m, n, w, static_cast<int64_t *>(e)); break;
+        case 1: voronoi_kernel<D, signed char, FULL><<<blocks, 128, 0, st>>>(m, n, w, static_cast<signed char *>(e)); break;
+        case 2: voronoi_kernel<D, short, FULL><<<blocks, 128, 0, st>>>(m, n, w, static_cast<short *>(e)); break;
+        case 4: voronoi_kernel<D, int, FULL><<<blocks, 128, 0, st>>>(m, n, w, static_cast<int *>(e)); break;
+        default: voronoi_kernel<D, long long, FULL><<<blocks, 128, 0, st>>>(m, n, w, static_cast<long long *>(e)); break;
     }
 }
 
@@ -1000,6 +1009,9 @@ int agd_prep_batch(const agd_batch_prep *p, agd_stream_t stream) {
     A.seed_index = p->seed_index;
     A.geom = p->geom;
     A.rhs = p->rhs;
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < D; ++i)
     A.values = p->values;
     A.bits = reinterpret_cast<unsigned *>(p->seedbits);
     A.bad = p->bad_seed;
@@ -1030,6 +1042,22 @@ int agd_prep_walls(int ndim, const int *shape, const int *shape_i, const uint8_t
     if ((ndim != 2 && ndim != 3) || !shape || !shape_i || !geo_of(ndim, shape, shape_i, g) || (g.size_tot % 32) != 0 ||
         !walls || !wall_dist || !tmp || bound < 0 || bound > 254)
         return set_error(AGD_STATUS_INVALID, "agd_prep_walls: bad arguments (bound in [0, 254])");
+static int voronoi(int ndim, const float *m, long long n, float *weights, void *offsets, int offset_bytes, bool full,
+                   cudaStream_t st) {
+    if (ndim < 1 || ndim > 3 || n < 0 || (n > 0 && (!m || !weights || !offsets)) ||
+        (offset_bytes != 1 && offset_bytes != 2 && offset_bytes != 4 && offset_bytes != 8))
+        return set_error(AGD_STATUS_INVALID, "agd_voronoi_decomposition: bad arguments (ndim 1 to 3, "
+                                             "offset_bytes 1, 2, 4 or 8)");
+    if (n == 0) return AGD_STATUS_OK;
+    if (ndim == 1) launch_voronoi<1, false>(m, n, weights, offsets, offset_bytes, st);
+    else if (ndim == 2 && full) launch_voronoi<2, true>(m, n, weights, offsets, offset_bytes, st);
+    else if (ndim == 2) launch_voronoi<2, false>(m, n, weights, offsets, offset_bytes, st);
+    else if (full) launch_voronoi<3, true>(m, n, weights, offsets, offset_bytes, st);
+    else launch_voronoi<3, false>(m, n, weights, offsets, offset_bytes, st);
+    const cudaError_t err = cudaGetLastError();
+    return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("voronoi_decomposition", err);
+}
+
     cudaStream_t st = (cudaStream_t)stream;
     // _SetGeometry.py:271-277: 0 at walls, `bound` passes of the L1 kernel, cut beyond `bound`
     const int rc = distance_map(ndim, shape, walls, bound, bound, true, tmp, tmp + g.n, st);
@@ -1059,17 +1087,13 @@ int agd_prep_walls_batch(int ndim, const int *shape, const int *shape_i, int n, 
 int agd_voronoi_decomposition(int ndim, const float *m, long long n, float *weights, void *offsets, int offset_bytes,
                               agd_stream_t stream) {
     clear_error();
-    if (ndim < 1 || ndim > 3 || n < 0 || (n > 0 && (!m || !weights || !offsets)) ||
-        (offset_bytes != 1 && offset_bytes != 2 && offset_bytes != 4 && offset_bytes != 8))
-        return set_error(AGD_STATUS_INVALID, "agd_voronoi_decomposition: bad arguments (ndim 1 to 3, "
-                                             "offset_bytes 1, 2, 4 or 8)");
-    if (n == 0) return AGD_STATUS_OK;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (ndim == 1) launch_voronoi<1>(m, n, weights, offsets, offset_bytes, st);
-    else if (ndim == 2) launch_voronoi<2>(m, n, weights, offsets, offset_bytes, st);
-    else launch_voronoi<3>(m, n, weights, offsets, offset_bytes, st);
-    const cudaError_t err = cudaGetLastError();
-    return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("voronoi_decomposition", err);
+    return voronoi(ndim, m, n, weights, offsets, offset_bytes, false, (cudaStream_t)stream);
+}
+
+int agd_voronoi_matrices(int ndim, const float *m, long long n, float *weights, void *offsets, int offset_bytes,
+                         agd_stream_t stream) {
+    clear_error();
+    return voronoi(ndim, m, n, weights, offsets, offset_bytes, true, (cudaStream_t)stream);
 }
 
 int agd_selling(int ndim, const float *m, int n, float *weights, int32_t *offsets, agd_stream_t stream) {

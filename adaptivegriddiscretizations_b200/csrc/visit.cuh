@@ -120,8 +120,8 @@ __global__ void stencil_kernel(const Inst *insts, int ninst, int total_tiles, Ct
             const long long n_t = base + n0 + 32 * q;
             float w[SD];
             int e[SD][3];
-            if (D == 2) selling2(m[q], w, e);
-            else selling3(m[q], w, e);
+            if (D == 2) selling2_fast(m[q], w, e);
+            else selling3_fast(m[q], w, e);
 #pragma unroll
             for (int r = 0; r < SD; ++r) {
                 int word = 0;

@@ -328,6 +328,11 @@ int agd_flow(const agd_instance *inst, float *flow_vector, float *flow_weightsum
 
 /* Distance-to-seed map in 1/5 pixel units, saturated at 255, grid layout
  * (inf_convolution with a 3^ndim kernel, ceil(target_tolerance) passes, cut
+/* agd_voronoi_decomposition of whole matrices m (ndim, ndim, n), of which the lower
+ * triangle is read. */
+int agd_voronoi_matrices(int ndim, const float *m, long long n, float *weights, void *offsets, int offset_bytes,
+                         agd_stream_t stream);
+
  * beyond 5*target_tolerance: agd/Eikonal/HFM_CUDA/_GetGeodesics.py:51-75).
  * seed_mask: grid layout uint8.  tmp: scratch of the same size. */
 int agd_eucl_map(int ndim, const int *shape, const uint8_t *seed_mask, int npasses, int cut,
