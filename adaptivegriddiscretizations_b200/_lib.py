@@ -103,17 +103,19 @@ SIGNATURES = {
     "agd_block_expand": (_I, [_I, _P, _P, _I, _P, _I, ctypes.c_float, _P, _P]),
     "agd_block_squeeze": (_I, [_I, _P, _P, _I, _P, _P, _P]),
     "agd_prep_seeds": (_I, [_I, _P, _P, _P, _P, _I, _P, _P, _P, _P]),
+    "agd_prep_args": (_I, [_I, _P, _P, _P, _I, _P, _P, _P, _I, _P, _P, _P, _P]),
+    "agd_nan_sum": (_I, [_P, ctypes.c_longlong, _P, _P]),
     "agd_prep_batch": (_I, [_P, _P]),
     "agd_prep_walls": (_I, [_I, _P, _P, _P, _I, _P, _P, _P, _P, _P]),
     "agd_prep_walls_batch": (_I, [_I, _P, _P, _I, _P, _I, _P, _P, _P]),
     "agd_selling": (_I, [_I, _P, _I, _P, _P, _P]),
     "agd_voronoi_decomposition": (_I, [_I, _P, ctypes.c_longlong, _P, _P, _I, _P]),
-    "agd_flow": (_I, [_P, _P, _P, _P, _P, _P]),
-    "agd_eucl_map": (_I, [_I, _P, _P, _I, _I, _P, _P, _P]),
     "agd_voronoi_matrices": (_I, [_I, _P, ctypes.c_longlong, _P, _P, _I, _P]),
+    "agd_flow": (_I, [_P, _P, _P, _P, _P, _P]),
+    "agd_eucl_map_seeds": (_I, [_I, _P, _P, _I, _I, _I, _P, _P]),
+    "agd_eucl_map": (_I, [_I, _P, _P, _I, _I, _P, _P, _P]),
     "agd_geodesics": (_I, [_P, _P, _P, _P, _P, _I, ctypes.c_float, ctypes.c_float, _I, _I, _I, _I, _I, _P, _I,
                            _P, _P, _P]),
-    "agd_eucl_map_seeds": (_I, [_I, _P, _P, _I, _I, _I, _P, _P]),
     "agd_reverse_workspace_bytes": (ctypes.c_size_t, [_P]),
     "agd_reverse": (_I, [_P, _P, _P, _P, _P, _P, ctypes.c_float, ctypes.c_float, _P, ctypes.c_size_t, _P, _P,
                          _P]),

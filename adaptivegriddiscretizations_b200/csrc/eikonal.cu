@@ -440,6 +440,115 @@ __device__ __forceinline__ bool grid_coords(const Geo &g, long long n_t, int *x,
     return in;
 }
 
+// The layout kernels below take four points a thread, neighbours along the last
+// axis of a tile, in 32-bit arithmetic with shifts: tile sides that are powers of
+// two, the last one at least 4, and fewer than 2^31 points (four_points()).  A
+// point a thread with 64-bit divisions, as the kernels beside them for other
+// shapes have it, took 107 us for a plane of 201^3 points in either direction,
+// 105 us for its seed bits and 169 us for the dual metric of 200^3; four points
+// 13 to 29, 10 and 61 us.
+struct Geo4 {
+    int nd, shape[3], so[3], lsi[3], lsz;
+    unsigned size_tot, n;
+};
+static bool four_points(const Geo &g, Geo4 &q) {
+    if (g.size_tot >= (1ll << 31) || g.si[g.nd - 1] % 4) return false;
+    q.nd = g.nd;
+    q.lsz = 0;
+    for (int k = 0; k < 3; ++k) {
+        int l = 0;
+        while ((1 << l) < g.si[k]) ++l;
+        if ((1 << l) != g.si[k]) return false;
+        q.shape[k] = g.shape[k];
+        q.so[k] = g.so[k];
+        q.lsi[k] = l;
+        q.lsz += l;
+    }
+    q.size_tot = (unsigned)g.size_tot;
+    q.n = (unsigned)g.n;
+    return true;
+}
+
+// The points n_t .. n_t + 3 (n_t a multiple of 4): how many of them are in the grid
+// (from the first on), and the grid index of the first.
+__device__ __forceinline__ int four_coords(const Geo4 &g, unsigned n_t, unsigned &flat) {
+    unsigned n_o = n_t >> g.lsz, n_i = n_t & ((1u << g.lsz) - 1u);
+    int x[3] = {0, 0, 0};
+#pragma unroll
+    for (int k = 2; k >= 0; --k) {
+        if (k >= g.nd) continue;
+        const unsigned q = k == 0 ? 0u : n_o / (unsigned)g.so[k];
+        x[k] = (int)(((n_o - q * g.so[k]) << g.lsi[k]) + (n_i & ((1u << g.lsi[k]) - 1u)));
+        n_o = q;
+        n_i >>= g.lsi[k];
+    }
+    bool in = true;
+    flat = 0;
+    int left = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (k >= g.nd) continue;
+        flat = flat * g.shape[k] + x[k];
+        left = g.shape[k] - x[k];
+        in = in && left > 0;
+    }
+    return in ? min(left, 4) : 0;
+}
+
+// block_expand: grid.y is the plane.  Vector loads where the rows allow them.
+__global__ void __launch_bounds__(256) expand4_kernel(Geo4 g, const float *__restrict__ src, int bcast, float pad, int wide,
+                                                      float *__restrict__ dst) {
+    const unsigned n_t = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (n_t >= g.size_tot) return;
+    unsigned flat;
+    const int c = four_coords(g, n_t, flat);
+    float v[4] = {pad, pad, pad, pad};
+    if (bcast) {
+        const float b = __ldg(src + blockIdx.y);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = j < c ? b : pad;
+    } else {
+        const float *p = src + (size_t)blockIdx.y * g.n + flat;
+        if (wide && c == 4) {
+            const float4 w = __ldg(reinterpret_cast<const float4 *>(p));
+            v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < c) v[j] = __ldg(p + j);
+        }
+    }
+    *reinterpret_cast<float4 *>(dst + (size_t)blockIdx.y * g.size_tot + n_t) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+__global__ void __launch_bounds__(256) squeeze4_kernel(Geo4 g, const float *__restrict__ src, int wide, float *__restrict__ dst) {
+    const unsigned n_t = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (n_t >= g.size_tot) return;
+    unsigned flat;
+    const int c = four_coords(g, n_t, flat);
+    if (c == 0) return;
+    const float4 w = __ldg(reinterpret_cast<const float4 *>(src + (size_t)blockIdx.y * g.size_tot + n_t));
+    float *p = dst + (size_t)blockIdx.y * g.n + flat;
+    if (wide && c == 4) {
+        *reinterpret_cast<float4 *>(p) = w;
+    } else {
+        const float v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < c) p[j] = v[j];
+    }
+}
+
+// Seed bits of a grid without seeds: the padding's.
+__global__ void __launch_bounds__(256) seedbits4_kernel(Geo4 g, unsigned *__restrict__ bits) {
+    const unsigned n_t = 4u * (blockIdx.x * blockDim.x + threadIdx.x);  // (whole warps: size_tot is a multiple of 32)
+    unsigned flat, word = 0;
+    if (n_t < g.size_tot) word = ((0xfu << four_coords(g, n_t, flat)) & 0xfu) << (n_t & 31u);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) word |= __shfl_xor_sync(kFull, word, o);
+    if (n_t < g.size_tot && (n_t & 31u) == 0u) bits[n_t >> 5] = word;
+}
+
 __global__ void block_expand_kernel(Geo g, int nplanes, const float *src, int bcast, float pad, float *dst) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= g.size_tot * nplanes) return;
@@ -517,6 +626,118 @@ __global__ void prep_geom_kernel(Geo g, const float *metric, int bcast, int is_d
     float out[6];
     geom_at(g.nd, bcast ? metric : metric + flat * sd, is_dual, h, out);
     for (int c = 0; c < sd; ++c) geom[c * g.size_tot + n_t] = out[c];
+}
+
+// The solver's arrays of one instance in one launch: values +inf, the right-hand
+// side (cost, or 1), the seed bits and the seeds, given by value (bilevel
+// indices, in order: a later duplicate wins).
+constexpr int kArgSeeds = 32;
+struct ArgSeeds {
+    int n, at[kArgSeeds];
+    float host_value[kArgSeeds];
+    const float *value;  // device values, or NULL: host_value
+};
+__global__ void __launch_bounds__(256) prep_args4_kernel(Geo4 g, const __grid_constant__ ArgSeeds seeds,
+                                                         const float *__restrict__ cost, int bcast, int wide,
+                                                         float *__restrict__ values, float *__restrict__ rhs,
+                                                         unsigned *__restrict__ bits) {
+    const unsigned n_t = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+    const bool on = n_t < g.size_tot;
+    unsigned word = 0;
+    if (on) {
+        unsigned flat;
+        const int c = four_coords(g, n_t, flat);
+        float v[4];
+        if (!cost || bcast) {
+            const float b = cost ? __ldg(cost) : 1.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = j < c ? b : finf();
+        } else if (wide && c == 4) {
+            const float4 w = __ldg(reinterpret_cast<const float4 *>(cost + flat));
+            v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = j < c ? __ldg(cost + flat + j) : finf();
+        }
+        unsigned nib = (0xfu << c) & 0xfu;
+        for (int s = 0; s < seeds.n; ++s) {
+            const unsigned at = (unsigned)seeds.at[s];
+            if ((at ^ n_t) & ~3u) continue;
+            const float x = seeds.value ? __ldg(seeds.value + s) : seeds.host_value[s];
+            nib |= 1u << (at & 3u);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = (at & 3u) == j ? x : v[j];
+        }
+        *reinterpret_cast<float4 *>(rhs + n_t) = make_float4(v[0], v[1], v[2], v[3]);
+        if (values) *reinterpret_cast<float4 *>(values + n_t) = make_float4(finf(), finf(), finf(), finf());
+        word = nib << (n_t & 31u);
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) word |= __shfl_xor_sync(kFull, word, o);
+    if (on && (n_t & 31u) == 0u) bits[n_t >> 5] = word;
+}
+
+// Sum (double) and number of the values that are not NaN, added to out.
+__global__ void __launch_bounds__(256) nan_sum_kernel(const float *__restrict__ x, long long n, double *out) {
+    double s = 0.0, c = 0.0;
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += gridDim.x * 256ll) {
+        const float v = __ldg(x + i);
+        if (v == v) {
+            s += v;
+            c += 1.0;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(kFull, s, o);
+        c += __shfl_xor_sync(kFull, c, o);
+    }
+    __shared__ double part[2][8];
+    if ((threadIdx.x & 31) == 0) {
+        part[0][threadIdx.x >> 5] = s;
+        part[1][threadIdx.x >> 5] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double t = 0.0;
+        for (int k = 0; k < 8; ++k) t += part[threadIdx.x][k];
+        atomicAdd(out + threadIdx.x, t);
+    }
+}
+
+template <int D>
+__global__ void __launch_bounds__(256) prep_geom4_kernel(Geo4 g, const float *__restrict__ metric, int bcast, int is_dual,
+                                                         float h0, float h1, float h2, int wide, float *__restrict__ geom) {
+    constexpr int SD = D * (D + 1) / 2;
+    const unsigned n_t = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (n_t >= g.size_tot) return;
+    unsigned flat;
+    const int c = four_coords(g, n_t, flat);
+    const float h[3] = {h0, h1, h2};
+    float m[4 * SD], out[SD][4];
+    if (bcast) {
+#pragma unroll
+        for (int i = 0; i < 4 * SD; ++i) m[i] = __ldg(metric + i % SD);
+    } else if (wide && c == 4) {  // the four points' metrics are 4 SD consecutive floats
+#pragma unroll
+        for (int i = 0; i < SD; ++i) {
+            const float4 w = __ldg(reinterpret_cast<const float4 *>(metric + (size_t)flat * SD) + i);
+            m[4 * i] = w.x; m[4 * i + 1] = w.y; m[4 * i + 2] = w.z; m[4 * i + 3] = w.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4 * SD; ++i) m[i] = i < c * SD ? __ldg(metric + (size_t)flat * SD + i) : 1.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float o[6];
+        geom_at(D, m + j * SD, is_dual, h, o);
+#pragma unroll
+        for (int k = 0; k < SD; ++k) out[k][j] = j < c ? o[k] : finf();
+    }
+#pragma unroll
+    for (int k = 0; k < SD; ++k)
+        *reinterpret_cast<float4 *>(geom + (size_t)k * g.size_tot + n_t) = make_float4(out[k][0], out[k][1], out[k][2], out[k][3]);
 }
 
 // Diagonal model: the squared dual costs 1/(c_k h_k)^2 of metric.with_costs(h)
@@ -788,6 +1009,9 @@ __global__ void voronoi_kernel(const float *__restrict__ m, long long n, float *
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         float mm[SD], ww[SD];
         int ee[SD][3];
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < D; ++i)
 #pragma unroll
             for (int j = 0; j <= i; ++j, ++c) mm[c] = __ldg(m + (FULL ? i * D + j : c) * n + p);
         if constexpr (D == 1) {
@@ -818,6 +1042,22 @@ static void launch_voronoi(const float *m, long long n, float *w, void *e, int o
     }
 }
 
+static int voronoi(int ndim, const float *m, long long n, float *weights, void *offsets, int offset_bytes, bool full,
+                   cudaStream_t st) {
+    if (ndim < 1 || ndim > 3 || n < 0 || (n > 0 && (!m || !weights || !offsets)) ||
+        (offset_bytes != 1 && offset_bytes != 2 && offset_bytes != 4 && offset_bytes != 8))
+        return set_error(AGD_STATUS_INVALID, "agd_voronoi_decomposition: bad arguments (ndim 1 to 3, "
+                                             "offset_bytes 1, 2, 4 or 8)");
+    if (n == 0) return AGD_STATUS_OK;
+    if (ndim == 1) launch_voronoi<1, false>(m, n, weights, offsets, offset_bytes, st);
+    else if (ndim == 2 && full) launch_voronoi<2, true>(m, n, weights, offsets, offset_bytes, st);
+    else if (ndim == 2) launch_voronoi<2, false>(m, n, weights, offsets, offset_bytes, st);
+    else if (full) launch_voronoi<3, true>(m, n, weights, offsets, offset_bytes, st);
+    else launch_voronoi<3, false>(m, n, weights, offsets, offset_bytes, st);
+    const cudaError_t err = cudaGetLastError();
+    return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("voronoi_decomposition", err);
+}
+
 __global__ void selling_kernel(int nd, const float *m, int n, float *w, int *e) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
@@ -836,6 +1076,7 @@ __global__ void selling_kernel(int nd, const float *m, int n, float *w, int *e) 
 }
 
 static inline unsigned blocks_for(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
+static bool on16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace agd
 
@@ -899,6 +1140,16 @@ int agd_prep_geom(int ndim, const int *shape, const int *shape_i, const float *m
     Geo g;
     if (ndim < 2 || !geo_of(ndim, shape, shape_i, g) || !metric || !geom || !grid_scales)
         return set_error(AGD_STATUS_INVALID, "agd_prep_geom: bad arguments");
+    Geo4 q;
+    if (four_points(g, q) && on16(geom)) {
+        const int wide = g.shape[ndim - 1] % 4 == 0 && on16(metric);
+        const float h0 = (float)grid_scales[0], h1 = (float)grid_scales[1], h2 = ndim == 3 ? (float)grid_scales[2] : 1.f;
+        const unsigned nb = blocks_for(g.size_tot / 4, 256);
+        if (ndim == 2) prep_geom4_kernel<2><<<nb, 256, 0, (cudaStream_t)stream>>>(q, metric, broadcast, is_dual, h0, h1, h2, wide, geom);
+        else prep_geom4_kernel<3><<<nb, 256, 0, (cudaStream_t)stream>>>(q, metric, broadcast, is_dual, h0, h1, h2, wide, geom);
+        const cudaError_t err = cudaGetLastError();
+        return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("prep_geom", err);
+    }
     prep_geom_kernel<<<blocks_for(g.size_tot, 256), 256, 0, (cudaStream_t)stream>>>(
         g, metric, broadcast, is_dual, grid_scales[0], grid_scales[1], ndim == 3 ? grid_scales[2] : 1.0, geom);
     const cudaError_t err = cudaGetLastError();
@@ -936,8 +1187,15 @@ int agd_block_expand(int ndim, const int *shape, const int *shape_i, int nplanes
     Geo g;
     if (!geo_of(ndim, shape, shape_i, g) || nplanes < 1 || !src || !dst)
         return set_error(AGD_STATUS_INVALID, "agd_block_expand: bad arguments");
-    block_expand_kernel<<<blocks_for(g.size_tot * nplanes, 256), 256, 0, (cudaStream_t)stream>>>(
-        g, nplanes, src, src_broadcast, pad, dst);
+    Geo4 q;
+    if (four_points(g, q) && on16(dst) && nplanes <= 65535) {
+        const int wide = g.shape[ndim - 1] % 4 == 0 && on16(src);
+        expand4_kernel<<<dim3(blocks_for(g.size_tot / 4, 256), nplanes), 256, 0, (cudaStream_t)stream>>>(q, src, src_broadcast, pad,
+                                                                                                        wide, dst);
+    } else {
+        block_expand_kernel<<<blocks_for(g.size_tot * nplanes, 256), 256, 0, (cudaStream_t)stream>>>(
+            g, nplanes, src, src_broadcast, pad, dst);
+    }
     const cudaError_t err = cudaGetLastError();
     return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("block_expand", err);
 }
@@ -948,7 +1206,13 @@ int agd_block_squeeze(int ndim, const int *shape, const int *shape_i, int nplane
     Geo g;
     if (!geo_of(ndim, shape, shape_i, g) || nplanes < 1 || !src || !dst)
         return set_error(AGD_STATUS_INVALID, "agd_block_squeeze: bad arguments");
-    block_squeeze_kernel<<<blocks_for(g.n * nplanes, 256), 256, 0, (cudaStream_t)stream>>>(g, nplanes, src, dst);
+    Geo4 q;
+    if (four_points(g, q) && on16(src) && nplanes <= 65535) {
+        const int wide = g.shape[ndim - 1] % 4 == 0 && on16(dst);
+        squeeze4_kernel<<<dim3(blocks_for(g.size_tot / 4, 256), nplanes), 256, 0, (cudaStream_t)stream>>>(q, src, wide, dst);
+    } else {
+        block_squeeze_kernel<<<blocks_for(g.n * nplanes, 256), 256, 0, (cudaStream_t)stream>>>(g, nplanes, src, dst);
+    }
     const cudaError_t err = cudaGetLastError();
     return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("block_squeeze", err);
 }
@@ -960,7 +1224,10 @@ int agd_prep_seeds(int ndim, const int *shape, const int *shape_i, const int32_t
     if (!geo_of(ndim, shape, shape_i, g) || n < 0 || (n > 0 && !seed_index) || (g.size_tot % 32) != 0)
         return set_error(AGD_STATUS_INVALID, "agd_prep_seeds: bad arguments");
     cudaStream_t st = (cudaStream_t)stream;
-    if (seedbits)
+    Geo4 q;
+    if (seedbits && four_points(g, q))
+        seedbits4_kernel<<<blocks_for(g.size_tot / 4, 256), 256, 0, st>>>(q, reinterpret_cast<unsigned *>(seedbits));
+    else if (seedbits)
         seedbits_init_kernel<<<blocks_for(g.size_tot / 32, 256), 256, 0, st>>>(g, reinterpret_cast<unsigned *>(seedbits));
     if (trigger) cudaMemsetAsync(trigger, 0, (size_t)(g.size_tot / g.size_i), st);
     if (n > 0) {
@@ -969,6 +1236,49 @@ int agd_prep_seeds(int ndim, const int *shape, const int *shape_i, const int32_t
     }
     const cudaError_t err = cudaGetLastError();
     return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("prep_seeds", err);
+}
+
+int agd_prep_args(int ndim, const int *shape, const int *shape_i, const float *cost, int cost_broadcast,
+                  const int32_t *seed_index, const float *seed_host_values, const float *seed_values, int nseeds,
+                  float *values, float *rhs, uint8_t *seedbits, agd_stream_t stream) {
+    clear_error();
+    Geo g;
+    Geo4 q;
+    if ((ndim != 2 && ndim != 3) || !shape || !shape_i || !geo_of(ndim, shape, shape_i, g) || (g.size_tot % 32) != 0 ||
+        nseeds < 0 || (nseeds > 0 && (!seed_index || (!seed_values && !seed_host_values))) || !rhs || !seedbits)
+        return set_error(AGD_STATUS_INVALID, "agd_prep_args: bad arguments");
+    if (nseeds > kArgSeeds || !four_points(g, q) || !on16(rhs) || (values && !on16(values)))
+        return set_error(AGD_STATUS_UNSUPPORTED, "agd_prep_args: more than 32 seeds, or not a built tile shape");
+    ArgSeeds a;
+    a.n = nseeds;
+    a.value = seed_values;
+    for (int s = 0; s < nseeds; ++s) {
+        int n_o = 0, n_i = 0;
+        for (int k = 0; k < ndim; ++k) {
+            const int x = seed_index[s * ndim + k];
+            if (x < 0 || x >= shape[k]) return set_error(AGD_STATUS_INVALID, "agd_prep_args: seed outside the grid");
+            n_o = n_o * g.so[k] + x / g.si[k];
+            n_i = n_i * g.si[k] + x % g.si[k];
+        }
+        a.at[s] = n_o * g.size_i + n_i;
+        a.host_value[s] = seed_host_values ? seed_host_values[s] : 0.f;
+    }
+    const int wide = g.shape[ndim - 1] % 4 == 0 && on16(cost);
+    prep_args4_kernel<<<blocks_for(g.size_tot / 4, 256), 256, 0, (cudaStream_t)stream>>>(
+        q, a, cost, cost_broadcast, wide, values, rhs, reinterpret_cast<unsigned *>(seedbits));
+    const cudaError_t err = cudaGetLastError();
+    return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("prep_args", err);
+}
+
+int agd_nan_sum(const float *x, long long n, double *out, agd_stream_t stream) {
+    clear_error();
+    if (!x || !out || n < 0) return set_error(AGD_STATUS_INVALID, "agd_nan_sum: bad arguments");
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t err = cudaMemsetAsync(out, 0, 2 * sizeof(double), st);
+    if (err != cudaSuccess) return set_cuda_error("nan_sum", err);
+    if (n > 0) nan_sum_kernel<<<(unsigned)std::min<long long>((n + 2047) / 2048, 148 * 4), 256, 0, st>>>(x, n, out);
+    err = cudaGetLastError();
+    return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("nan_sum", err);
 }
 
 int agd_prep_batch(const agd_batch_prep *p, agd_stream_t stream) {
@@ -1009,9 +1319,6 @@ int agd_prep_batch(const agd_batch_prep *p, agd_stream_t stream) {
     A.seed_index = p->seed_index;
     A.geom = p->geom;
     A.rhs = p->rhs;
-        int c = 0;
-#pragma unroll
-        for (int i = 0; i < D; ++i)
     A.values = p->values;
     A.bits = reinterpret_cast<unsigned *>(p->seedbits);
     A.bad = p->bad_seed;
@@ -1042,22 +1349,6 @@ int agd_prep_walls(int ndim, const int *shape, const int *shape_i, const uint8_t
     if ((ndim != 2 && ndim != 3) || !shape || !shape_i || !geo_of(ndim, shape, shape_i, g) || (g.size_tot % 32) != 0 ||
         !walls || !wall_dist || !tmp || bound < 0 || bound > 254)
         return set_error(AGD_STATUS_INVALID, "agd_prep_walls: bad arguments (bound in [0, 254])");
-static int voronoi(int ndim, const float *m, long long n, float *weights, void *offsets, int offset_bytes, bool full,
-                   cudaStream_t st) {
-    if (ndim < 1 || ndim > 3 || n < 0 || (n > 0 && (!m || !weights || !offsets)) ||
-        (offset_bytes != 1 && offset_bytes != 2 && offset_bytes != 4 && offset_bytes != 8))
-        return set_error(AGD_STATUS_INVALID, "agd_voronoi_decomposition: bad arguments (ndim 1 to 3, "
-                                             "offset_bytes 1, 2, 4 or 8)");
-    if (n == 0) return AGD_STATUS_OK;
-    if (ndim == 1) launch_voronoi<1, false>(m, n, weights, offsets, offset_bytes, st);
-    else if (ndim == 2 && full) launch_voronoi<2, true>(m, n, weights, offsets, offset_bytes, st);
-    else if (ndim == 2) launch_voronoi<2, false>(m, n, weights, offsets, offset_bytes, st);
-    else if (full) launch_voronoi<3, true>(m, n, weights, offsets, offset_bytes, st);
-    else launch_voronoi<3, false>(m, n, weights, offsets, offset_bytes, st);
-    const cudaError_t err = cudaGetLastError();
-    return err == cudaSuccess ? AGD_STATUS_OK : set_cuda_error("voronoi_decomposition", err);
-}
-
     cudaStream_t st = (cudaStream_t)stream;
     // _SetGeometry.py:271-277: 0 at walls, `bound` passes of the L1 kernel, cut beyond `bound`
     const int rc = distance_map(ndim, shape, walls, bound, bound, true, tmp, tmp + g.n, st);

@@ -922,14 +922,18 @@ static __global__ void setup_tiles(Sched S, int total_tiles) {
             for (int j = 0; j < (I.size_i >> 5); ++j) any |= __ldg(bits + j);
             active = any != 0;
         } else {
-            for (int n_i = 0; n_i < I.size_i && !active; ++n_i) {
-                int q = n_i;
+            // row after row along the last axis (at most 16 bits, inside one word):
+            // the bits of its points inside the grid
+            const int last = I.a.ndim - 1, len = I.a.shape_i[last];
+            const int valid = min(len, I.a.shape[last] - xo[last] * len);
+            for (int n_i = 0; n_i < I.size_i && !active; n_i += len) {
+                int q = n_i / len;
                 bool in = true;
-                for (int k = I.a.ndim - 1; k >= 0; --k) {
+                for (int k = last - 1; k >= 0; --k) {
                     in = in && xo[k] * I.a.shape_i[k] + q % I.a.shape_i[k] < I.a.shape[k];
                     q /= I.a.shape_i[k];
                 }
-                active = in && ((__ldg(bits + (n_i >> 5)) >> (n_i & 31)) & 1u);
+                active = in && ((__ldg(bits + (n_i >> 5)) >> (n_i & 31)) & ((1u << valid) - 1u)) != 0u;
             }
         }
     }

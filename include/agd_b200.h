@@ -234,6 +234,21 @@ int agd_prep_seeds(int ndim, const int *shape, const int *shape_i, const int32_t
                    const float *seed_values, int n, float *rhs, uint8_t *seedbits, uint8_t *trigger,
                    agd_stream_t stream);
 
+/* The solver's arrays of one instance in one launch (agd_block_expand and
+ * agd_prep_seeds of a cold start): rhs = cost (device, grid layout; NULL: 1;
+ * cost_broadcast != 0: one value) with +inf padding, the seeds' values there and
+ * their bits, values = +inf (NULL: not written).  seed_index: HOST, (nseeds,
+ * ndim), inside the grid, at most 32; their values on the device (seed_values)
+ * or, where that is NULL, on the host.  AGD_STATUS_UNSUPPORTED for more seeds or
+ * a tile shape that is not built: then the separate calls. */
+int agd_prep_args(int ndim, const int *shape, const int *shape_i, const float *cost, int cost_broadcast,
+                  const int32_t *seed_index, const float *seed_host_values, const float *seed_values, int nseeds,
+                  float *values, float *rhs, uint8_t *seedbits, agd_stream_t stream);
+
+/* out[0] = the sum, out[1] = the number of the n values of x that are not NaN
+ * (device, double). */
+int agd_nan_sum(const float *x, long long n, double *out, agd_stream_t stream);
+
 /* Preparation of n instances that share one grid and tile shape, for repeated
  * batched solves: one launch writes, for every instance, the geometry (as
  * agd_prep_geom, agd_prep_geom_diagonal or agd_prep_geom_rander), the
@@ -313,6 +328,11 @@ int agd_selling(int ndim, const float *m, int n, float *weights, int32_t *offset
 int agd_voronoi_decomposition(int ndim, const float *m, long long n, float *weights, void *offsets,
                               int offset_bytes, agd_stream_t stream);
 
+/* agd_voronoi_decomposition of whole matrices m (ndim, ndim, n), of which the lower
+ * triangle is read. */
+int agd_voronoi_matrices(int ndim, const float *m, long long n, float *weights, void *offsets, int offset_bytes,
+                         agd_stream_t stream);
+
 /* ------------------------------------------------------------------- flow -- */
 
 /* Upwind geodesic flow of a solved instance, one pass over all tiles (the
@@ -328,15 +348,16 @@ int agd_flow(const agd_instance *inst, float *flow_vector, float *flow_weightsum
 
 /* Distance-to-seed map in 1/5 pixel units, saturated at 255, grid layout
  * (inf_convolution with a 3^ndim kernel, ceil(target_tolerance) passes, cut
-/* agd_voronoi_decomposition of whole matrices m (ndim, ndim, n), of which the lower
- * triangle is read. */
-int agd_voronoi_matrices(int ndim, const float *m, long long n, float *weights, void *offsets, int offset_bytes,
-                         agd_stream_t stream);
-
  * beyond 5*target_tolerance: agd/Eikonal/HFM_CUDA/_GetGeodesics.py:51-75).
  * seed_mask: grid layout uint8.  tmp: scratch of the same size. */
 int agd_eucl_map(int ndim, const int *shape, const uint8_t *seed_mask, int npasses, int cut,
                  uint8_t *eucl, uint8_t *tmp, agd_stream_t stream);
+
+/* agd_eucl_map of a few seeds given by their grid indices ((nseeds, ndim) int32,
+ * those outside the grid ignored): the same map, by the costs of the shortest
+ * paths in a box around each seed instead of passes over the grid. */
+int agd_eucl_map_seeds(int ndim, const int *shape, const int32_t *seed_index, int nseeds, int npasses, int cut,
+                       uint8_t *eucl, agd_stream_t stream);
 
 /* Geodesic backtracking, one warp per tip, with the reference's chunking
  * (chunks of `typical_len` points restarting the stopping-criteria history,
@@ -357,12 +378,6 @@ int agd_geodesics(const agd_instance *inst, const float *flow_vector, const floa
 
 /* Workspace for agd_reverse. */
 size_t agd_reverse_workspace_bytes(const agd_instance *inst);
-
-/* agd_eucl_map of a few seeds given by their grid indices ((nseeds, ndim) int32,
- * those outside the grid ignored): the same map, by the costs of the shortest
- * paths in a box around each seed instead of passes over the grid. */
-int agd_eucl_map_seeds(int ndim, const int *shape, const int32_t *seed_index, int nseeds, int npasses, int cut,
-                       uint8_t *eucl, agd_stream_t stream);
 
 /* Reverse-mode sensitivity: solves diag*lam - W^T lam = sens on the tiles, where
  * W holds the upwind flow weights (flow_weights/flow_indices of agd_flow) and
