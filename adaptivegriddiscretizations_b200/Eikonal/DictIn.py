@@ -199,6 +199,15 @@ class dictIn(MutableMapping):
             return dev
         return value
 
+    def __contains__(self, key):
+        if key in _singleIn:  # (through __getitem__: an error unless there is one value)
+            try:
+                self[key]
+            except KeyError:
+                return False
+            return True
+        return key in self.store  # without reading the value: a deferred array stays on the host
+
     def raw(self, key):
         """The stored value without moving a deferred host array to the device:
         a device tensor, or a float32 numpy array for small host-side arrays."""
@@ -275,9 +284,9 @@ class dictIn(MutableMapping):
 
     @property
     def gridScales(self):
-        if "gridScales" in self:
+        if "gridScales" in self.store:
             return self.host("gridScales").astype(np.float32)
-        return np.full(self.vdim, float(self.host("gridScale")), np.float32)
+        return np.array([float(self.host("gridScale"))] * self.vdim, np.float32)
 
     @property
     def corners(self):

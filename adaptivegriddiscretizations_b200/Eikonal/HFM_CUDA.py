@@ -197,6 +197,7 @@ def _submit_uniform(hfmIns, launch):
         itf.SetKernelTraits()
         itf.SetGeometry()
         itf.SetArgs()
+        itf.atol  # noqa: B018  (the default tolerance's record)
         itf.PostProcess()
         itf.SolveAD()
         itf.GetGeodesics()
@@ -414,21 +415,26 @@ class Interface:
     # ------------------------------------------------------------- keys ---
     def HasValue(self, key):
         self.hfmOut["keys"]["visited"].append(key)
-        return key in self.hfmIn
+        return key in self.hfmIn.store
 
-    def GetValue(self, key, default="_None", verbosity=2, array_float=False, help="Sorry : no help for this key"):
-        """Value of a key, with the reference's bookkeeping (_Interface.py:80-122)."""
-        assert key not in self.hfmOut["keys"]["help"]
-        self.hfmOut["keys"]["help"][key] = help
-        self.hfmOut["keys"]["default"][key] = default
-        if key in self.hfmIn:
-            self.hfmOut["keys"]["used"].append(key)
-            value = self.hfmIn[key]
+    def GetValue(self, key, default="_None", verbosity=2, array_float=False, help="Sorry : no help for this key",
+                 host=False):
+        """Value of a key, with the reference's bookkeeping (_Interface.py:80-122).
+        host: a value that the host holds stays there (a scalar or a small array that is only
+        read on the host); a device tensor is returned as it is."""
+        keys = self.hfmOut["keys"]
+        assert key not in keys["help"]
+        keys["help"][key] = help
+        keys["default"][key] = default
+        if key in self.hfmIn.store:
+            keys["used"].append(key)
+            value = self.hfmIn.raw(key) if host else self.hfmIn[key]
             if array_float is False:
                 return value
-            value = _to_tensor(value)
+            if not host:
+                value = _to_tensor(value)
             if isinstance(array_float, tuple):
-                shapeRef, shape = array_float, tuple(value.shape)
+                shapeRef, shape = array_float, tuple(np.shape(value))
                 if len(shapeRef) != len(shape):
                     raise ValueError(f"Field {key} has incorrect number of dimensions. "
                                      f"Expected shape {shapeRef}, found {shape}")
@@ -445,7 +451,7 @@ class Interface:
                     print(f"see out['keys']['default'][{key}] for default")
                 else:
                     print(f"key {key} defaults to {default}")
-            if isinstance(default, numbers.Number) and array_float is not False:
+            if isinstance(default, numbers.Number) and array_float is not False and not host:
                 default = _to_tensor(default)
             return default
 
@@ -563,9 +569,10 @@ class Interface:
         self.size_o = int(np.prod(self.shape_o))
         self.size_tot = self.size_o * self.size_i
         if "gridScale" in self.hfmIn:
-            self.GetValue("gridScale", help="Scale of the computational grid")
+            self.GetValue("gridScale", help="Scale of the computational grid", host=True)
         else:
-            self.GetValue("gridScales", array_float=(self.ndim,), help="Axis independent scales of the computational grid")
+            self.GetValue("gridScales", array_float=(self.ndim,), host=True,
+                          help="Axis independent scales of the computational grid")
         self.h = np.asarray(self.hfmIn.gridScales, np.float32).reshape(-1)
         self.c_shape = (ctypes.c_int * 3)(*self.shape, *([1] * (3 - self.ndim)))
         self.c_shape_i = (ctypes.c_int * 3)(*self.shape_i, *([1] * (3 - self.ndim)))
@@ -659,23 +666,27 @@ class Interface:
             if cv.dim() != self.ndim + 1 or tuple(cv.shape[:-1]) != self.shape:
                 raise ValueError(f"costVariation has shape {tuple(cv.shape)}; expected {self.shape} + (n,)")
         self.costVariation = cv
+        self._mean = None  # the mean cost on its way to the host, when the default tolerance needs it
         if self.HasValue("atol") and self.HasValue("rtol"):
             tol = None
         else:
-            tol = self.GetValue("tol", default="_Dummy", array_float=tuple(),
+            tol = self.GetValue("tol", default="_Dummy", array_float=tuple(), host=True,
                                 help="Convergence tolerance for the fixed point solver (determines atol, rtol)")
             if isinstance(tol, str) and tol == "_Dummy":
-                if mean_cost is None:
-                    mean_cost = float(torch.nanmean(cost.float())) if cost.dim() else float(cost)
-                tol = np.float32(mean_cost * _FLOAT_RES * 5.0)
-                self.hfmOut["keys"]["default"]["tol"] = np.float32(tol)
+                if mean_cost is None and cost.dim():
+                    self._mean = _start_mean(cost, self.stream)
+                    tol = self._default_tol() if self.verbosity >= 2 else None
+                else:
+                    tol = np.float32((float(cost) if mean_cost is None else mean_cost) * _FLOAT_RES * 5.0)
+                    self.hfmOut["keys"]["default"]["tol"] = np.float32(tol)
             else:
-                tol = float(tol)
-        self.atol = float(self.GetValue("atol", default=tol, array_float=tuple(),
-                                        help="Absolute convergence tolerance for the fixed point solver"))
-        self.rtol = float(self.GetValue("rtol", default=0.0 if self.multiprecision else _FLOAT_RES * 5.0,
-                                        array_float=tuple(),
-                                        help="Relative convergence tolerance for the fixed point solver"))
+                tol = _scalar32(tol)
+        atol = self.GetValue("atol", default=tol, array_float=tuple(), host=True,
+                             help="Absolute convergence tolerance for the fixed point solver")
+        self._atol = None if atol is None else _scalar32(atol)  # None: five resolutions of the mean cost, read later
+        self.rtol = _scalar32(self.GetValue("rtol", default=0.0 if self.multiprecision else _FLOAT_RES * 5.0,
+                                            array_float=tuple(), host=True,
+                                            help="Relative convergence tolerance for the fixed point solver"))
         if self.multiprecision:
             # a power of two well below the grid scale (_SetGeometry.py:52-56)
             hmin = float(np.min(self.h))
@@ -697,6 +708,35 @@ class Interface:
                 raise ValueError("wallDistBound must lie in [0, 254]")
             self.wall_dist = torch.empty(self.size_tot, dtype=torch.uint8, device="cuda")
 
+    def _default_tol(self):
+        """The default tolerance, from the mean cost (waits for its reduction only)."""
+        buf, event = self._mean
+        event.synchronize()
+        total, count = buf.tolist()
+        tol = np.float32((total / count if count else math.nan) * _FLOAT_RES * 5.0)
+        self.hfmOut["keys"]["default"]["tol"] = tol
+        return tol
+
+    @property
+    def atol(self):
+        if self._atol is None:
+            tol = self._default_tol()
+            self.hfmOut["keys"]["default"]["atol"] = tol
+            self._atol = float(tol)
+        return self._atol
+
+    @atol.setter
+    def atol(self, value):
+        self._atol = value
+
+    @property
+    def seed_idx_t(self):
+        """Grid indices of the seeds, (n, ndim) int32 on the device."""
+        if self._seed_idx_t is None:
+            self._seed_idx_t = torch.from_numpy(self.seedIndices.astype(np.int32)).pin_memory().to(
+                "cuda", non_blocking=True)
+        return self._seed_idx_t
+
     def SetArgs(self):
         """Initial values, rhs, seeds (agd/Eikonal/HFM_CUDA/_SetArgs.py:8-177)."""
         L = _lib.lib()
@@ -707,9 +747,7 @@ class Interface:
             help="Visit every tile at the first iteration (for warm starts from an upper bound of the "
                  "solution; by default only the tiles holding seeds are active at first)"))
         self.values_t = torch.empty(self.size_tot, dtype=torch.float32, device="cuda")
-        if values is None:
-            self.values_t.fill_(math.inf)
-        else:
+        if values is not None:
             v = values.contiguous().float()
             _lib.check(L.agd_block_expand(self.ndim, self.c_shape, self.c_shape_i, 1, _lib.ptr(v), 0,
                                           ctypes.c_float(math.inf), _lib.ptr(self.values_t), self.stream),
@@ -721,11 +759,7 @@ class Interface:
             self.values_next_t = torch.empty_like(self.values_t)
             self.valuesq_next_t = torch.empty_like(self.valuesq_t)
         self.rhs_t = torch.empty(self.size_tot, dtype=torch.float32, device="cuda")
-        c = self.cost.contiguous()
-        _lib.check(L.agd_block_expand(self.ndim, self.c_shape, self.c_shape_i, 1, _lib.ptr(c.reshape(-1)),
-                                      1 if c.dim() == 0 else 0, ctypes.c_float(math.inf), _lib.ptr(self.rhs_t),
-                                      self.stream), "rhs")
-        seeds = self.GetValue("seeds", default=None, array_float=(-1, self.ndim),
+        seeds = self.GetValue("seeds", default=None, array_float=(-1, self.ndim), host=True,
                               help="Points from where the front propagation starts")
         self.reverseAD = self.HasValue("sensitivity")
         if seeds is None:
@@ -769,10 +803,24 @@ class Interface:
         self.nseeds_in = len(ci)
         self.seedIndices = idx
         self.seed_values = seedValues.contiguous().float()
-        self.seed_idx_t = torch.from_numpy(idx.astype(np.int32)).pin_memory().to("cuda", non_blocking=True)
+        self._seed_idx_t = None
         self.seedbits = torch.empty(self.size_tot // 8, dtype=torch.uint8, device="cuda")
         # with walls, the first tiles are those of the seeds alone (_SetArgs.py:119-126)
         self.trigger_t = None if self.walls is None else torch.zeros(self.size_o, dtype=torch.uint8, device="cuda")
+        c = self.cost.contiguous()
+        new_values = self.values_t if values is None else None  # (+inf)
+        if len(idx) <= 32 and self.walls is None and self.size_tot < 1 << 31:  # everything in one launch, the seeds by value
+            idx32 = np.ascontiguousarray(idx, np.int32)
+            _lib.check(L.agd_prep_args(self.ndim, self.c_shape, self.c_shape_i, _lib.ptr(c), int(c.dim() == 0),
+                                       idx32.ctypes.data_as(ctypes.c_void_p), None, _lib.ptr(self.seed_values), len(idx),
+                                       _lib.ptr(new_values), _lib.ptr(self.rhs_t), _lib.ptr(self.seedbits),
+                                       self.stream), "args")
+            return
+        if new_values is not None:
+            new_values.fill_(math.inf)
+        _lib.check(L.agd_block_expand(self.ndim, self.c_shape, self.c_shape_i, 1, _lib.ptr(c.reshape(-1)),
+                                      1 if c.dim() == 0 else 0, ctypes.c_float(math.inf), _lib.ptr(self.rhs_t),
+                                      self.stream), "rhs")
         _lib.check(L.agd_prep_seeds(self.ndim, self.c_shape, self.c_shape_i, _lib.ptr(self.seed_idx_t),
                                     _lib.ptr(self.seed_values), len(idx), _lib.ptr(self.rhs_t),
                                     _lib.ptr(self.seedbits), _lib.ptr(self.trigger_t), self.stream), "seeds")
@@ -948,16 +996,18 @@ class Interface:
         try:
             nbytes = L.agd_plan_workspace_bytes(plan)
             ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
-            stats = torch.zeros(2, dtype=torch.int64, device="cuda")
+            stats = torch.empty(2, dtype=torch.int64, device="cuda")  # written by the solve
+            stats_host = torch.empty(2, dtype=torch.int64, pin_memory=True)
             _lib.check(L.agd_plan_upload(plan, _lib.ptr(ws), nbytes, self.stream), "upload")
             start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             start.record()
             _lib.check(L.agd_plan_run(plan, _lib.ptr(ws), nbytes, _lib.ptr(stats), None, self.stream), "solve")
             stop.record()
-            stop.synchronize()
+            stats_host.copy_(stats, non_blocking=True)
+            torch.cuda.current_stream().synchronize()  # one wait for the solve and its statistics
         finally:
             L.agd_plan_destroy(plan)
-        s = stats.cpu().numpy()
+        s = stats_host.numpy()
         niter_o = int(s[0] & 0xffffffff)
         status = int((s[0] >> 32) & 0xffffffff)
         self.tile_visits = int(s[1])
@@ -1231,6 +1281,24 @@ class Interface:
         self.hfmOut["keys"]["unused"] = list(set(self.hfmIn.keys()) - set(self.hfmOut["keys"]["used"]))
         if self.verbosity >= 1 and self.hfmOut["keys"]["unused"]:
             print(f"!! Warning !! Unused keys from user : {self.hfmOut['keys']['unused']}")
+
+
+def _scalar32(x):
+    """A scalar option as the float of its float32 value."""
+    return float(x) if isinstance(x, torch.Tensor) else float(np.float32(x))
+
+
+def _start_mean(cost, stream):
+    """Queues the sum and the number of the cost's values that are not NaN and their copy to
+    page-locked memory: (the copy, the event after it)."""
+    c = cost.contiguous()
+    dev = torch.empty(2, dtype=torch.float64, device="cuda")
+    _lib.check(_lib.lib().agd_nan_sum(_lib.ptr(c), c.numel(), _lib.ptr(dev), stream), "mean cost")
+    host = torch.empty(2, dtype=torch.float64, pin_memory=True)
+    host.copy_(dev, non_blocking=True)
+    event = torch.cuda.Event()
+    event.record()
+    return host, event
 
 
 def _host_scalar(x):

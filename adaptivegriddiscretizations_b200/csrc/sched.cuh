@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <vector>
 
@@ -197,7 +198,7 @@ struct Ctrl {
     unsigned long long pad[14], round[2][16];
 };
 
-// Workspace: [Inst][InstState][tile_inst][lists][flags][score0][score1][queue][Ctrl][stats]
+// Workspace: [Inst][tile_inst][lists][queue][flags][bits][score0][score1][InstState][Ctrl][stats][stencil]
 struct WsLayout {
     size_t inst, istate, tile_inst, lists, flags, bits, score0, score1, queue, ctrl, stats, stencil, total;
     int total_tiles;
@@ -254,15 +255,15 @@ static bool layout(const agd_instance *a, int n, WsLayout &L, Inst *out, bool st
     const unsigned qcap = (unsigned)(2 * tiles + 10 * kMaxWarps) | 1u;  // odd: see kSlotEmpty
     size_t off = 0;
     L.inst = off; off = align256(off + sizeof(Inst) * n);
-    L.istate = off; off = align256(off + sizeof(InstState) * n);
     L.tile_inst = off; off = align256(off + sizeof(int) * tiles);
     L.nlists = gated ? kMaxLists : 2;
     L.lists = off; off = align256(off + sizeof(int) * tiles * L.nlists);
-    L.flags = off; off = align256(off + sizeof(unsigned) * tiles);
+    L.queue = off; off = align256(off + sizeof(unsigned long long) * qcap);
+    L.flags = off; off = align256(off + sizeof(unsigned) * tiles);  // from here to the stencil: cleared by a launch
     L.bits = off; off = align256(off + sizeof(unsigned) * bitmap_words(tiles));
     L.score0 = off; off = align256(off + sizeof(unsigned) * tiles);
     L.score1 = off; off = align256(off + sizeof(unsigned) * tiles);
-    L.queue = off; off = align256(off + sizeof(unsigned long long) * qcap);
+    L.istate = off; off = align256(off + sizeof(InstState) * n);
     L.ctrl = off; off = align256(off + sizeof(Ctrl));
     L.stats = off; off = align256(off + sizeof(agd_stats) * n);
     L.stencil = off; off = align256(off + sizeof(float) * stencil_floats);
@@ -1024,15 +1025,23 @@ template <class Visitor>
 static int rounds_ctas(int total_tiles, const agd_launch *cfg, int *ctas) {
     auto kern = rounds_worker<Visitor>;
     constexpr int smem = (int)sizeof(typename Visitor::RoundSmem) * (Visitor::kRoundWarps / Visitor::kRoundG);
-    int dev = 0, nsm = 0, per_sm = 0;
+    int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return set_cuda_error("cudaGetDevice");
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return set_cuda_error("rounds shared memory");
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Visitor::kRoundWarps * 32, smem) != cudaSuccess)
-        return set_cuda_error("occupancy query");
-    if (per_sm < 1) return set_error(AGD_STATUS_UNSUPPORTED, "rounds kernel does not fit on an SM");
-    const int most = std::min(per_sm * nsm, kMaxRoundCtas);
+    // the kernel's resident CTAs and the SMs of a device do not change: asked once (low 16 bits: SMs)
+    static std::atomic<int> known[64];
+    int k = dev >= 0 && dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (k == 0) {
+        int nsm = 0, per_sm = 0;
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+            return set_cuda_error("rounds shared memory");
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Visitor::kRoundWarps * 32, smem) != cudaSuccess)
+            return set_cuda_error("occupancy query");
+        if (per_sm < 1) return set_error(AGD_STATUS_UNSUPPORTED, "rounds kernel does not fit on an SM");
+        k = per_sm << 16 | nsm;
+        if (dev >= 0 && dev < 64) known[dev].store(k, std::memory_order_relaxed);
+    }
+    const int nsm = k & 0xffff, most = std::min((k >> 16) * nsm, kMaxRoundCtas);
     int c = cfg && cfg->ctas > 0 ? cfg->ctas : total_tiles <= 16 * nsm ? nsm : most;
     *ctas = std::max(1, std::min(std::min(c, most), total_tiles));
     return AGD_STATUS_OK;
@@ -1091,9 +1100,8 @@ static int run_sched(const WsLayout &L, void *ws, int n, const typename Visitor:
         S.bitmap = kPushRounds;
         S.rctas = (unsigned)ctas;
         S.rwords = (unsigned)(((L.total_tiles + ctas - 1) / ctas + 31) / 32);
-        err = cudaMemsetAsync(w + L.istate, 0, sizeof(InstState) * n, st);
-        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.bits, 0, L.queue - L.bits, st);
-        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.ctrl, 0, L.stencil - L.ctrl, st);
+        // bitmaps, scores, control block and stats; the stencil region after them is written in full by the stencil pass
+        err = cudaMemsetAsync(w + L.bits, 0, L.stencil - L.bits, st);
         if (err != cudaSuccess) return set_cuda_error("workspace clear", err);
         if ((err = Visitor::prepare(S, L, st)) != cudaSuccess) return set_cuda_error("prepare", err);
         setup_tiles<<<(L.total_tiles + 255) / 256, 256, 0, st>>>(S, L.total_tiles);
@@ -1109,11 +1117,9 @@ static int run_sched(const WsLayout &L, void *ws, int n, const typename Visitor:
         // Bitmap pushes for launches of many instances: the pushes of a visit then
         // wait for nothing, and an epoch is published in tile order.
         S.bitmap = (L.nlists == 2 && n >= kPairInstances) ? kPushBits : kPushLists;
-        err = cudaMemsetAsync(w + L.istate, 0, sizeof(InstState) * n, st);
-        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.flags, 0, L.queue - L.flags, st);
-        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.queue, 0xff, L.ctrl - L.queue, st);
-        // control block and stats; the stencil region after them is written in full by the stencil pass
-        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.ctrl, 0, L.stencil - L.ctrl, st);
+        err = cudaMemsetAsync(w + L.queue, 0xff, L.flags - L.queue, st);
+        // flags to stats; the stencil region after them is written in full by the stencil pass
+        if (err == cudaSuccess) err = cudaMemsetAsync(w + L.flags, 0, L.stencil - L.flags, st);
         if (err != cudaSuccess) return set_cuda_error("workspace clear", err);
         if ((err = Visitor::prepare(S, L, st)) != cudaSuccess) return set_cuda_error("prepare", err);
         setup_tiles<<<(L.total_tiles + 255) / 256, 256, 0, st>>>(S, L.total_tiles);
