@@ -203,6 +203,7 @@ struct WsLayout {
     size_t inst, istate, tile_inst, lists, flags, bits, score0, score1, queue, ctrl, stats, stencil, total;
     int total_tiles;
     int nlists;  // epoch lists per instance (2, or kMaxLists with release epochs)
+    int same;    // tiles of every instance, 0 if they differ
     unsigned qcap;
 };
 
@@ -245,6 +246,7 @@ static bool layout(const agd_instance *a, int n, WsLayout &L, Inst *out, bool st
             I.stencil_off = stencil_floats;  // the pointer is set once the workspace is known
             stencil_floats += 2ll * (a[i].ndim * (a[i].ndim + 1) / 2) * I.size_tot;
         }
+        L.same = i == 0 || L.same == I.size_o ? I.size_o : 0;
         tiles += I.size_o;
         if (tiles > 0x3fffffff) return false;
         if (out) out[i] = I;
@@ -315,6 +317,10 @@ struct Sched {
     // Rounds: tile t belongs to CTA t % rctas, as bit t / rctas of its rwords
     // words in the bitmap of its epoch's parity (rctas rwords words each).
     unsigned rctas, rwords;
+    // Instances of one size: tile t belongs to instance t / size, as the high word of
+    // t * div_m shifted by div_s (exact below 2^31; div_m 0: sizes differ).
+    unsigned div_m;
+    int div_s;
 };
 enum { kPushLists = 0, kPushBits = 1, kPushRounds = 2 };
 
@@ -689,7 +695,9 @@ __global__ void __launch_bounds__(WPB * 32, Visitor::kMinCtas * 4 / WPB) sched_w
         }
         prefetched = ahead;
         int ii;
-        if (inst_in_smem) {
+        if (S.div_m) {
+            ii = (int)(__umulhi(t, S.div_m) >> S.div_s);
+        } else if (inst_in_smem) {
             int lo = 0, hi = S.ninst - 1;
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
@@ -738,6 +746,12 @@ __global__ void __launch_bounds__(WPB * 32, Visitor::kMinCtas * 4 / WPB) sched_w
 //   static bool due(const Args&, int t, int e)
 // (kOrdered true): a tile pushed before it is due waits.
 constexpr int kRoundChunk = 64;  // words of own tiles listed at a time
+// Launches that run in rounds: fewer than kPairInstances instances, or up to
+// kRoundInstances whose tiles are at most kRoundTiles in all.  Rounds against the queue,
+// batches of Riemann2: 200 of 100^2 (34 k tiles) 1.86 / 2.65 ms, 32 of 512^2 (131 k)
+// 5.8 / 8.0, 64 of 512^2 (262 k) 10.2 / 11.2, 256 of 256^2 (262 k) 9.7 / 8.4, 128 of
+// 512^2 (524 k) 18.9 / 15.9: with many tiles an instance need not wait for the others.
+constexpr int kRoundInstances = 512, kRoundTiles = 1 << 17;
 
 // Barrier of a group of G warps, and its vote.  Groups of several warps use a
 // named barrier (1 + the group's index in the CTA: at most 15 such groups).
@@ -772,8 +786,8 @@ __global__ void __launch_bounds__(Visitor::kRoundWarps * 32, Visitor::kRoundCtas
     __shared__ int s_list[kRoundChunk * 32];
     __shared__ int s_next[NG];
     __shared__ int s_n, s_take, s_pushed, s_go;
-    __shared__ int s_base[kPairInstances], s_max[kPairInstances], s_flags[kPairInstances], s_last[kPairInstances];
-    __shared__ unsigned s_visits[kPairInstances];
+    __shared__ int s_base[kRoundInstances], s_max[kRoundInstances], s_flags[kRoundInstances], s_last[kRoundInstances];
+    __shared__ unsigned s_visits[kRoundInstances];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = warp / G, gtid = tid - group * (32 * G);
     for (int i = tid; i < S.ninst; i += NW * 32) {
@@ -1078,6 +1092,14 @@ static Sched sched_at(const WsLayout &L, void *ws, int ninst) {
     S.ctrl = reinterpret_cast<Ctrl *>(w + L.ctrl);
     S.stats = reinterpret_cast<agd_stats *>(w + L.stats);
     S.ninst = ninst;
+    S.div_m = 0;
+    S.div_s = 0;
+    if (L.same > 1) {  // div_m = ceil(2^(31 + l) / size) with 2^(l - 1) < size <= 2^l
+        int l = 1;
+        while ((1ll << l) < L.same) ++l;
+        S.div_m = (unsigned)(((1ull << (31 + l)) + L.same - 1) / L.same);
+        S.div_s = l - 1;
+    }
     S.nwarps = 0;
     S.tgroup = 1;
     S.timeout_ns = 2000000000ull;
@@ -1093,7 +1115,8 @@ static int run_sched(const WsLayout &L, void *ws, int n, const typename Visitor:
     if (cfg && cfg->timeout_ns > 0) S.timeout_ns = (unsigned long long)cfg->timeout_ns;
     cudaError_t err;
     char *w = static_cast<char *>(ws);
-    if (Visitor::kQueueless || (n < kPairInstances && L.nlists == 2)) {
+    const bool few = n < kPairInstances || (n <= kRoundInstances && L.total_tiles <= kRoundTiles);
+    if (Visitor::kQueueless || (few && L.nlists == 2)) {
         int ctas = 0;
         const int rc = rounds_ctas<Visitor>(L.total_tiles, cfg, &ctas);
         if (rc != AGD_STATUS_OK) return rc;

@@ -105,7 +105,7 @@ __global__ void stencil_kernel(const Inst *insts, int ninst, int total_tiles, Ct
     if (!I.stencil) return;
     const long long base = (long long)(t - I.tile_base) * I.size_i;
     const float *__restrict__ geom = I.a.geom;
-    float *__restrict__ out = I.stencil;
+    float *__restrict__ out = I.stencil + 2 * SD * base;  // the tile's planes, one after the other
     // two points of the lane per step, their loads issued together
     for (int n0 = lane; n0 < I.size_i; n0 += 64) {
         float m[2][SD];
@@ -117,7 +117,6 @@ __global__ void stencil_kernel(const Inst *insts, int ninst, int total_tiles, Ct
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             if (n0 + 32 * q >= I.size_i) break;
-            const long long n_t = base + n0 + 32 * q;
             float w[SD];
             int e[SD][3];
             if (D == 2) selling2_fast(m[q], w, e);
@@ -126,8 +125,8 @@ __global__ void stencil_kernel(const Inst *insts, int ninst, int total_tiles, Ct
             for (int r = 0; r < SD; ++r) {
                 int word = 0;
                 if (!pack_offset<D>(e[r], word)) atomicOr(&ctrl->err, (unsigned)AGD_STATUS_UNSUPPORTED);
-                __stcs(out + (size_t)r * I.size_tot + n_t, w[r]);
-                __stcs(out + (size_t)(SD + r) * I.size_tot + n_t, __int_as_float(word));
+                __stcs(out + r * I.size_i + n0 + 32 * q, w[r]);
+                __stcs(out + (SD + r) * I.size_i + n0 + 32 * q, __int_as_float(word));
             }
         }
     }
@@ -158,7 +157,7 @@ __global__ void stencil_walls_kernel(const Inst *insts, int ninst, int total_til
             ri /= I.a.shape_i[k];
         }
         for (int r = 0; r < SD; ++r) {
-            float *slot = I.stencil + (size_t)(SD + r) * I.size_tot + n_t;
+            float *slot = I.stencil + 2 * SD * base + (SD + r) * I.size_i + n_i;
             const int word = __float_as_int(*slot);
             int e[3] = {0, 0, 0};
             unpack_offset<D>(word, e);
@@ -228,9 +227,14 @@ struct Visit {
     __device__ __forceinline__ static bool greater(float u, int uq, float v, int vq, float step) {
         return u - v > (float)(vq - uq) * step;
     }
-    __device__ __forceinline__ static void normalize(float &u, int &uq, float umax, float step) {
+    // inv: 1 / step where that is exact (step a power of two, as _SetGeometry.py:52-56
+    // chooses it), so that the quotient is a product; else 0.
+    __device__ __forceinline__ static float exact_inverse(float step) {
+        return (__float_as_uint(step) & 0x7fffffu) == 0u && step >= 0x1p-100f && step <= 0x1p100f ? 1.f / step : 0.f;
+    }
+    __device__ __forceinline__ static void normalize(float &u, int &uq, float umax, float step, float inv) {
         if (u < umax) {
-            const int n = (int)(u / step);
+            const int n = (int)(inv != 0.f ? u * inv : u / step);
             u -= (float)n * step;
             uq += n;
         }
@@ -314,7 +318,7 @@ struct Visit {
     // Grid point yt seen from point xt of a tile: inside the tile (li: its index
     // there), inside the grid (n_t: its bilevel index; any value otherwise).
     // The tile sides are equal powers of two, so one mask tests all the axes.
-    __device__ __forceinline__ static void locate(const agd_instance &A, const Inst &I, const int *xt, const int *yt,
+    __device__ __forceinline__ static void locate(const int *shape, const int *shape_o, const int *xt, const int *yt,
                                                   bool &intile, bool &indom, int &li, unsigned &n_t) {
         constexpr unsigned SM = TL::S0 - 1;
         static_assert(TL::S0 == TL::S1 && (D == 2 || TL::S0 == TL::S2) && (TL::S0 & SM) == 0, "cubic tiles");
@@ -324,8 +328,8 @@ struct Visit {
         for (int c = 0; c < D; ++c) {
             const unsigned y = (unsigned)yt[c];
             diff |= y ^ (unsigned)xt[c];
-            indom = indom && y < (unsigned)A.shape[c];
-            n_o = n_o * (unsigned)I.shape_o[c] + y / TL::S0;
+            indom = indom && y < (unsigned)shape[c];
+            n_o = n_o * (unsigned)shape_o[c] + y / TL::S0;
             n_i = n_i * TL::S0 + (y & SM);
         }
         intile = (diff & ~SM) == 0u;
@@ -339,7 +343,8 @@ struct Visit {
     // weights), then the weights and offsets (unpacked, or by Selling's
     // decomposition; unit offsets for Isotropic and Diagonal).
     static constexpr int kRaw = MODEL == AGD_MODEL_ISOTROPIC ? 1 : (MODEL == AGD_MODEL_DIAGONAL ? D : 2 * SD + (kDrift ? D : 0));
-    __device__ __forceinline__ static void stencil_load(const Inst &I, size_t n_t, float *raw) {
+    __device__ __forceinline__ static void stencil_load(const Inst &I, size_t base, int n_i, float *raw) {
+        const size_t n_t = base + n_i;
         if constexpr (MODEL == AGD_MODEL_ISOTROPIC) return;
         if constexpr (MODEL == AGD_MODEL_DIAGONAL) {
 #pragma unroll
@@ -348,7 +353,7 @@ struct Visit {
         }
         if (I.stencil) {
 #pragma unroll
-            for (int r = 0; r < 2 * SD; ++r) raw[r] = __ldg(I.stencil + (size_t)r * I.size_tot + n_t);
+            for (int r = 0; r < 2 * SD; ++r) raw[r] = __ldg(I.stencil + 2 * SD * base + n_i + r * TL::SIZE);
         } else {
 #pragma unroll
             for (int c = 0; c < SD; ++c) raw[c] = __ldg(I.a.geom + (size_t)c * I.size_tot + n_t);
@@ -402,7 +407,7 @@ struct Visit {
     __device__ __forceinline__ static void stencil(const Inst &I, size_t n_t, float *w, int (*e)[3]) {
         float raw[kRaw];
         unsigned hide[NACT];
-        stencil_load(I, n_t, raw);
+        stencil_load(I, n_t, 0, raw);  // (no cache: planes over the whole grid)
         stencil_decode(I, raw, w, e, hide);
     }
 
@@ -412,14 +417,24 @@ struct Visit {
         const agd_instance &A = I.a;
         const int lane = tid & 31;
         const bool lead = G == 1 || tid < 32;  // the first warp does the tile's bookkeeping
+        // (in registers: after a volatile access the compiler would read the descriptor again)
+        int shape[D], shape_o[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            shape[k] = A.shape[k];
+            shape_o[k] = I.shape_o[k];
+        }
+        const int niter_i = A.niter_i;
         int xo[3] = {0, 0, 0};
         {
             int r = n_o;
 #pragma unroll
-            for (int k = D - 1; k >= 0; --k) {
-                xo[k] = r % I.shape_o[k];
-                r /= I.shape_o[k];
+            for (int k = D - 1; k > 0; --k) {
+                const int q = r / shape_o[k];
+                xo[k] = r - q * shape_o[k];
+                r = q;
             }
+            xo[0] = r;
         }
         // Scores of this tile and of its neighbours at epoch e-1 (complete): loaded
         // now, so that their latency overlaps the visit (cuda/Propagation.h:103-167).
@@ -430,11 +445,11 @@ struct Visit {
             y[lane >> 1] += 2 * (lane & 1) - 1;
             bool ok = true;
 #pragma unroll
-            for (int k = 0; k < D; ++k) ok = ok && y[k] >= 0 && y[k] < I.shape_o[k];
+            for (int k = 0; k < D; ++k) ok = ok && y[k] >= 0 && y[k] < shape_o[k];
             if (ok) {
                 int m = 0;
 #pragma unroll
-                for (int k = 0; k < D; ++k) m = m * I.shape_o[k] + y[k];
+                for (int k = 0; k < D; ++k) m = m * shape_o[k] + y[k];
                 nb = I.tile_base + m;
             }
         }
@@ -447,7 +462,7 @@ struct Visit {
         float *u_out = A.values;
         const int *q_in = nullptr;
         int *q_out = nullptr;
-        const float step = A.multip_step;
+        const float step = A.multip_step, umax = A.multip_max, inv = MP ? exact_inverse(step) : 0.f;
         if constexpr (MP) {
             const bool odd = (e & 1) != 0;
             u_in = odd ? A.values : A.values_next;
@@ -485,7 +500,7 @@ struct Visit {
             seed[p] = (__ldg(A.seedbits + (n_t >> 3)) >> (n_t & 7)) & 1;
             rhs[p] = __ldg(A.rhs + n_t);
             if constexpr (MP) qold[p] = __ldcg(q_in + n_t);
-            stencil_load(I, n_t, raw[p]);
+            stencil_load(I, base, point_of(tid, p), raw[p]);
         }
 #pragma unroll
         for (int p = 0; p < P; ++p) {
@@ -500,7 +515,7 @@ struct Visit {
                 if (seed[p]) {
                     u0 = rhs[p];
                     q0 = 0;
-                    normalize(u0, q0, A.multip_max, step);
+                    normalize(u0, q0, umax, step, inv);
                 }
                 us[n_i] = u0;
                 uqs[n_i] = q0;
@@ -521,8 +536,10 @@ struct Visit {
                 }
                 if constexpr (kDrift) drift_shifts(raw[p], ev, fsh[p]);
             }
-            // Addresses first, then every load, then the stores: a load followed by
-            // its own store would make the neighbours' L2 round trips serial.
+            // Addresses first, then every load of the point, then the stores: a load
+            // followed by its own store would make the neighbours' L2 round trips
+            // serial.  (The loads of a lane's two points together: the registers
+            // spill, batch 128 of Riemann2 512^2 15.2 -> 15.9 ms.)
             float out[kSlots ? NTOT : 1], out2[kSlots && ORD2 ? NTOT : 1];
 #pragma unroll
             for (int k = 0; k < NACT; ++k) {
@@ -539,7 +556,7 @@ struct Visit {
                         bool intile, indom;
 #pragma unroll
                         for (int c = 0; c < D; ++c) yt[c] = s ? xt[c] + (far + 1) * ev[k][c] : xt[c] - (far + 1) * ev[k][c];
-                        locate(A, I, xt, yt, intile, indom, li, n_t);
+                        locate(shape, shape_o, xt, yt, intile, indom, li, n_t);
                         if constexpr (kSlots) {
                             const bool in = intile && !hidden;
                             float v = finf();
@@ -584,7 +601,7 @@ struct Visit {
             }
         }
         gsync(group);
-        for (int it = 0; it < A.niter_i; ++it) {
+        for (int it = 0; it < niter_i; ++it) {
             bool moved = false;
             if constexpr (MP) {
                 // strict sweeps: every point from the state at the start of the sweep
@@ -644,7 +661,7 @@ struct Visit {
                     float c = hfm_update<NACT>(rhs[p], v, w);
                     int cq = vqmin;
                     if (c == finf()) cq = 0;
-                    else normalize(c, cq, A.multip_max, step);
+                    else normalize(c, cq, umax, step, inv);
                     cand[p] = c;
                     candq[p] = cq;
                 }
@@ -858,6 +875,12 @@ template <unsigned long long VMASK, int G>
 __device__ __forceinline__ bool dispatch(const Sched &S, int t, int ii, int e, int tid, int group, float *us) {
     const Inst &I = S.inst[ii];
     const int n_o = t - I.tile_base;
+    if constexpr ((VMASK & (VMASK - 1)) == 0) {  // one variant: no switch
+#define AGD_CASE(V, D, A, B, C, M, MP, F, O2, W) \
+    if constexpr (VMASK == (1ull << V)) return Visit<Tile<D, A, B, C>, M, MP, F, O2, W, G>::run(S, I, ii, n_o, e, tid, group, us);
+        AGD_VARIANTS(AGD_CASE)
+#undef AGD_CASE
+    }
     switch (I.variant) {
 #define AGD_CASE(V, D, A, B, C, M, MP, F, O2, W)                                                          \
     case V:                                                                                               \
@@ -898,12 +921,12 @@ struct EikonalVisitor {
     // Resident 4-warp CTAs per SM of the queue's workers that the register
     // budget must allow: 256-point tiles keep 8 points per lane in registers,
     // Riemann3 twelve neighbours per point, multiprecision an integer part
-    // beside every value.  Riemann2 8x8: 8 CTAs at up to 64 registers (batch 128
-    // of 512^2: +1 % over 9 CTAs at 56 registers, +7 % over 10 CTAs at 48).
+    // beside every value.  Riemann2 8x8: 7 CTAs at up to 72 registers (batch 128
+    // of 512^2: 15.2 ms against 15.4 at 8 CTAs and 64 registers).
     static constexpr int kMinCtas = (VMASK & kTiles16)                                            ? 4
                                     : (VMASK & kSelling3)                                         ? 5
                                     : (VMASK & (kMpVariants | kFactorVariants | kOrder2Variants)) ? 7
-                                    : (VMASK & (1ull << V_RIEM2_8))                               ? 8
+                                    : (VMASK & (1ull << V_RIEM2_8))                               ? 7
                                                                                                   : 9;
     struct Args {};
     struct Smem {
@@ -915,7 +938,14 @@ struct EikonalVisitor {
     // Rounds: groups of kRoundG warps per tile.
     static constexpr bool kQueueless = false;
     static constexpr bool kAll16 = (VMASK & ~kTiles16) == 0;
-    static constexpr int kRoundG = kAll16 ? ((VMASK & kOrder2Variants) ? 1 : 8) : 2;
+    // Isotropic and Diagonal 64-point tiles: a warp (Isotropic3 201^3: 4.1 ms against
+    // 5.3 with two: a visit has little to compute, and half of a group idles in
+    // each phase); Riemann: two, whose points' neighbours fit the registers then
+    // (Riemann3 200^3: 9.4 ms against 10.2; Riemann2 512^2 1.39 against 1.59 ms);
+    // 16x16 tiles alone in a kernel: eight, a point a thread.
+    static constexpr unsigned long long kUnit64 =
+        (1ull << V_ISO2_8) | (1ull << V_ISO3_4) | (1ull << V_DIAG2_8) | (1ull << V_DIAG3_4);
+    static constexpr int kRoundG = kAll16 ? ((VMASK & kOrder2Variants) ? 1 : 8) : (VMASK & ~kUnit64) ? 2 : 1;
     static constexpr int kRoundWarps = 16;
     static constexpr int kRoundCtas = 2;
     struct RoundSmem {
