@@ -472,6 +472,10 @@ struct Visit {
         }
         int *uqs = reinterpret_cast<int *>(us + TL::SIZE);  // integer parts, after the float parts
         float uold[P], rhs[P];
+        // A thread's own values stay in registers where there is one of them.
+        constexpr bool kOwn = P == 1;
+        float own = 0.f;
+        int ownq = 0;
         int qold[P];
         float wts[P][NACT];
         // Neighbour of each stencil offset.  With kSlots: the shared-memory address
@@ -519,8 +523,11 @@ struct Visit {
                 }
                 us[n_i] = u0;
                 uqs[n_i] = q0;
+                own = u0;
+                ownq = q0;
             } else {
-                us[n_i] = seed[p] ? rhs[p] : uold[p];
+                own = seed[p] ? rhs[p] : uold[p];
+                us[n_i] = own;
             }
             int ev[NACT][3];
             unsigned hide[NACT];
@@ -644,7 +651,7 @@ struct Visit {
                         // one outside carries it in its float part already
                         const int n_i = point_of(tid, p);
                         if (vqmin != kIntMax) {
-                            const float u0 = us[n_i] + (float)(uqs[n_i] - vqmin) * step;
+                            const float u0 = (kOwn ? own : us[n_i]) + (float)((kOwn ? ownq : uqs[n_i]) - vqmin) * step;
                             order2(u0, v, w, side, [&](int k, int sd) {
                                 const float x = nbv2[p][2 * k + sd];
                                 const int b = __float_as_int(x);
@@ -669,9 +676,9 @@ struct Visit {
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
                     const int n_i = point_of(tid, p);
-                    if (!seed[p] && greater(us[n_i], uqs[n_i], cand[p], candq[p], step)) {
-                        us[n_i] = cand[p];
-                        uqs[n_i] = candq[p];
+                    if (!seed[p] && greater(kOwn ? own : us[n_i], kOwn ? ownq : uqs[n_i], cand[p], candq[p], step)) {
+                        us[n_i] = own = cand[p];
+                        uqs[n_i] = ownq = candq[p];
                         moved = true;
                     }
                 }
@@ -706,7 +713,7 @@ struct Visit {
                             w[k] = wts[p][k];
                             if constexpr (ORD2) side[k] = a > b;
                         }
-                        if constexpr (ORD2) order2(us[n_i], v, w, side, [&](int k, int sd) {
+                        if constexpr (ORD2) order2(kOwn ? own : us[n_i], v, w, side, [&](int k, int sd) {
                             // (with factorisation, the shift of x +/- 2 e_k; outside the tile
                             // without slots nbv2 carries it already)
                             if constexpr (kSlots) {
@@ -727,8 +734,8 @@ struct Visit {
                     // a group they may read each other's new values (neighbours of one
                     // colour, Riemann offsets): either is a value of this sweep.
                     __syncwarp();
-                    if (mine && us[n_i] > cand) {
-                        us[n_i] = cand;
+                    if (mine && (kOwn ? own : us[n_i]) > cand) {
+                        us[n_i] = own = cand;
                         moved = true;
                     }
                     if (ph + 1 < NPH) gsync(group);
@@ -740,11 +747,11 @@ struct Visit {
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             const int n_i = point_of(tid, p);
-            const float u = us[n_i];
+            const float u = kOwn ? own : us[n_i];
             __stcg(u_out + base + n_i, u);
             float diff, uabs;
             if constexpr (MP) {
-                const int q = uqs[n_i];
+                const int q = kOwn ? ownq : uqs[n_i];
                 __stcg(q_out + base + n_i, q);
                 diff = fabsf(uold[p] - u + (float)(qold[p] - q) * step);  // Update.h:212-216
                 uabs = fabsf(u + (float)q * step);
@@ -946,8 +953,11 @@ struct EikonalVisitor {
     static constexpr unsigned long long kUnit64 =
         (1ull << V_ISO2_8) | (1ull << V_ISO3_4) | (1ull << V_DIAG2_8) | (1ull << V_DIAG3_4);
     static constexpr int kRoundG = kAll16 ? ((VMASK & kOrder2Variants) ? 1 : 8) : (VMASK & ~kUnit64) ? 2 : 1;
-    static constexpr int kRoundWarps = 16;
-    static constexpr int kRoundCtas = 2;
+    // A CTA of 16x16 tiles has the whole SM, 4 groups of 8 warps: with two CTAs of
+    // two groups, an epoch of few tiles more often gives one of them three
+    // (Isotropic2 1203x1501 float64: 4.7 ms, 4.1 with one).
+    static constexpr int kRoundWarps = kAll16 ? 32 : 16;
+    static constexpr int kRoundCtas = kAll16 ? 1 : 2;
     struct RoundSmem {
         float u[smem_floats<VMASK, kRoundG>()];
     };
