@@ -2042,7 +2042,7 @@ int conv_row(const agd_conv *c, const void *w, const float *bias, int relu, void
     void *out = out_bf16 ? out_bf16 : static_cast<void *>(out_f32);
     if (s0.up || (two_in && s1.up) || s0.channels % 32 || (two_in && s1.channels % 32) || c->cout % 32) return 0;
     // few channels at 128 columns are conv_halo's: 32 -> 32 of 128 problems 90 us
-    // there against 116 here, 32 -> 96 of 32 45 us against 88; 96 -> 32 233 us against 137
+    // there against 138 here, 96 -> 32 233 us against 210
     if (c->W == 128 && s0.channels + (two_in ? s1.channels : 0) < 96) return 0;
     if (c->W < 8 || c->W > 128 || 128 % c->W || c->H % (128 / c->W) || reinterpret_cast<uintptr_t>(out) % 16) return 0;
     RowArgs g{};
