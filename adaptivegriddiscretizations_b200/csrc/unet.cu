@@ -867,52 +867,43 @@ __global__ void __launch_bounds__(kHaloThreads, 1)
 // and the epilogue forms out[p] = D[p - 1, 0] + D[p, 1] + D[p + 1, 2], zero beyond a
 // row's ends (shuffles between the lanes, which are the pixels, and shared
 // memory between the warps).  A CTA tile is MT x 128 pixels, whole rows; per
-// block of 64 (32) channels one copy brings its rows and one above and below, and the
+// block of 32 channels one copy brings its rows and one above and below, and the
 // row taps dy are the same data W pixel rows further on, whole swizzle atoms.
 // Weights stay resident where they fit (they are then loaded once a CTA; with
-// several channel tiles, a CTA keeps to one of them), else a second ring brings
-// them per block and dy.  The copies are in rows of
-// 128 bytes where the channels allow (64 -> 64 channels at 64^2 60 us against 62,
-// 256 + 128 -> 128 at 32^2 93 against 125, 128 problems).
+// several channel tiles, a CTA keeps to one of them), else they come with each block.
 // Accumulators: double buffered, or two pixel tiles at once where the weights
 // are not resident, so that a block of them serves 256 pixels.
-// The issuing thread's own instructions count: with loops over blocks, taps and
-// tiles not unrolled it took 200 to 330 cycles per MMA, so all but the block are
-// template parameters (the 96 -> 32 layer at 128^2 343 -> 137 us).
-// Measured (128 problems), a load and an MMA per tap before: the layers at 64^2
-// and below 1265 -> 577 us, the 96 -> 32 layer at 128^2 233 -> 137 us.
+// Measured (128 problems): the 12 layers at 64^2 and below and the 96 -> 32 one at 128^2
+// 1475 -> 920 us, the forward 1.99 -> 1.31 ms.
 constexpr int kRowThreads = 320;   // a producer, an MMA and 2 x 4 epilogue warps
 constexpr int kRowStage = 32768;   // staging of the epilogue: 8 warps x 4 KB
 
 struct RowArgs {
     int H, W, rows;      // rows of a CTA tile (MT 128 / W)
-    int kb;              // channels of a block: 64 or 32
-    int nblk0, nblk;     // blocks of the first input, of both
+    int nblk0, nblk;     // 32-channel blocks of the first input, of both
     int cin, ct, ntiles; // input channels, output channels of a tile, channel tiles
-    int MT, nbuf, resident, slots, bslots;
+    int MT, nbuf, resident, slots;
     int ygroups, ptiles; // row groups of an image, pixel tiles of the launch
-    uint32_t a_bytes, b_bytes;  // a slot's rows, the weights of a block and dy
+    uint32_t a_bytes, b_bytes;  // a slot's rows, and the weights of a block (3 dy)
     const float *bias;
     int relu, f32, N;
     unsigned *err;
 };
 
-template <int KB, int MT, bool RES>
 __global__ void __launch_bounds__(kRowThreads, 1)
     conv_row_kernel(RowArgs g, const __grid_constant__ CUtensorMap xa0, const __grid_constant__ CUtensorMap xa1,
                     const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap omap) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ HaloPipe P;
-    __shared__ uint64_t bfull[8], bempty[8];
     __shared__ float edge[2][2][4][2][32];  // by group, parity of its chunk, warp: last pixel's D0 and first pixel's D2
     __shared__ __align__(16) float sbias[64];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t sbase = (umma::smem_u32(smem) + 1023u) & ~1023u;
     const uint32_t abase = sbase + kRowStage;
-    const uint32_t bbase = abase + g.slots * g.a_bytes;  // weights: all of them, or a ring
-    constexpr int row = 2 * KB;                           // bytes of a pixel's or a weight row's block
+    const uint32_t slot_bytes = g.a_bytes + (g.resident ? 0u : g.b_bytes);
+    const uint32_t rbase = abase + g.slots * slot_bytes;  // resident weights
     const int ncol = 3 * g.ct;                            // accumulator columns of a pixel tile
-    const uint32_t tcols = tmem_cols(g.nbuf * MT * ncol);
+    const uint32_t tcols = tmem_cols(g.nbuf * g.MT * ncol);
     // CTA c works on channel tile c % ntiles and every (grid / ntiles)-th pixel tile
     const int nt = blockIdx.x % g.ntiles, p0 = blockIdx.x / g.ntiles, pstep = gridDim.x / g.ntiles;
     const int ntl = p0 < g.ptiles && p0 < pstep ? (g.ptiles - p0 + pstep - 1) / pstep : 0;
@@ -925,10 +916,6 @@ __global__ void __launch_bounds__(kRowThreads, 1)
         for (int s = 0; s < g.slots; ++s) {
             umma::mbar_init(&P.full[s], 1);
             umma::mbar_init(&P.empty[s], 1);
-        }
-        for (int s = 0; s < g.bslots; ++s) {
-            umma::mbar_init(&bfull[s], 1);
-            umma::mbar_init(&bempty[s], 1);
         }
         for (int a = 0; a < 2; ++a) {
             umma::mbar_init(&P.accf[a], 1);
@@ -944,102 +931,71 @@ __global__ void __launch_bounds__(kRowThreads, 1)
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
-        // the weights of block b and dy: rows (dx, channel)
-        auto load_weights = [&](uint32_t dst, int b, int dy, uint64_t *bar) {
-            for (int dx = 0; dx < 3; ++dx)
-                tma_load_2d(dst + (uint32_t)(dx * g.ct * row), &wmap, (3 * dy + dx) * g.cin + KB * b, nt * g.ct, bar);
+        // the weights of block b: for each dy the rows (dx, channel) of 64 bytes
+        auto load_weights = [&](uint32_t dst, int b, uint64_t *bar) {
+            for (int tap = 0; tap < 9; ++tap)
+                tma_load_2d(dst + (uint32_t)(tap * g.ct) * 64u, &wmap, tap * g.cin + 32 * b, nt * g.ct, bar);
         };
-        if (lane == 0 && RES && ntl > 0) {
-            mbar_expect_tx(&P.bready, (uint32_t)(3 * g.nblk) * g.b_bytes);
-            for (int i = 0; i < 3 * g.nblk; ++i) load_weights(bbase + i * g.b_bytes, i / 3, i % 3, &P.bready);
+        if (lane == 0 && g.resident && ntl > 0) {
+            mbar_expect_tx(&P.bready, (uint32_t)g.nblk * g.b_bytes);
+            for (int b = 0; b < g.nblk; ++b) load_weights(rbase + b * g.b_bytes, b, &P.bready);
         }
         __syncwarp();
-        Ring R, RB;
-        bool wrapped = false, bwrapped = false, alive = true;
+        Ring R;
+        bool wrapped = false, alive = true;
         for (int tl = 0; tl < ntl && alive; ++tl) {
             const int t = p0 + tl * pstep, img = t / g.ygroups, y0 = (t - img * g.ygroups) * g.rows;
-            for (int b = 0; b < g.nblk && alive; ++b) {
+            for (int b = 0; b < g.nblk; ++b) {
                 if (wrapped && !mbar_wait_warp(&P.empty[R.s], R.ph ^ 1u, g.err, kWaitNs)) {
                     alive = false;
                     break;
                 }
                 if (lane == 0) {
-                    mbar_expect_tx(&P.full[R.s], g.a_bytes);
-                    tma_load_4d(abase + R.s * g.a_bytes, b < g.nblk0 ? &xa0 : &xa1,
-                                KB * (b < g.nblk0 ? b : b - g.nblk0), 0, y0 - 1, img, &P.full[R.s]);
+                    const uint32_t slot = abase + R.s * slot_bytes;
+                    mbar_expect_tx(&P.full[R.s], slot_bytes);
+                    tma_load_4d(slot, b < g.nblk0 ? &xa0 : &xa1, 32 * (b < g.nblk0 ? b : b - g.nblk0), 0, y0 - 1, img,
+                                &P.full[R.s]);
+                    if (!g.resident) load_weights(slot + g.a_bytes, b, &P.full[R.s]);
                 }
                 __syncwarp();
                 R.next(g.slots);
                 wrapped = wrapped || R.s == 0;
-                for (int dy = 0; dy < (RES ? 0 : 3); ++dy) {
-                    if (bwrapped && !mbar_wait_warp(&bempty[RB.s], RB.ph ^ 1u, g.err, kWaitNs)) {
-                        alive = false;
-                        break;
-                    }
-                    if (lane == 0) {
-                        mbar_expect_tx(&bfull[RB.s], g.b_bytes);
-                        load_weights(bbase + RB.s * g.b_bytes, b, dy, &bfull[RB.s]);
-                    }
-                    __syncwarp();
-                    RB.next(g.bslots);
-                    bwrapped = bwrapped || RB.s == 0;
-                }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA (lane 0 issues)
         const uint32_t idesc = umma::idesc_bf16(kBM, ncol, 0, 0);
-        const uint32_t dy_a = (uint32_t)(g.W * row) >> 4;
-        Ring R, RB;
-        bool ok = ntl > 0 && (!RES || mbar_wait_warp(&P.bready, 0, g.err, kWaitNs));
+        const uint64_t dy_a = (uint64_t)((uint32_t)g.W * 64u >> 4), dy_b = (uint64_t)((uint32_t)ncol * 64u >> 4);
+        Ring R;
+        bool ok = ntl > 0 && (!g.resident || mbar_wait_warp(&P.bready, 0, g.err, kWaitNs));
         int done = 0;
         for (int tl = 0; tl < ntl && ok; ++tl) {
             const int a = g.nbuf == 2 ? tl & 1 : 0, use = g.nbuf == 2 ? tl >> 1 : tl;  // the buffer's use-th tile
             if (use > 0 && !mbar_wait_warp(&P.acce[a], (use & 1) ^ 1, g.err, kWaitNs)) break;
             umma::tc_fence_after_sync();
-            const uint32_t d = P.taddr + (uint32_t)(a * MT * ncol);
+            const uint32_t d = P.taddr + (uint32_t)(a * g.MT * ncol);
             for (int b = 0; b < g.nblk; ++b) {
                 if (!mbar_wait_warp(&P.full[R.s], R.ph, g.err, kWaitNs)) {
                     ok = false;
                     break;
                 }
                 umma::tc_fence_after_sync();
-                // unrolled, one constant away from a base: the issue is else what bounds it
-                const uint64_t ad0 = swz_desc(abase + R.s * g.a_bytes, row);
-                auto issue = [&](uint64_t ad, uint64_t bd, bool add) {
+                if (lane == 0) {
+                    const uint32_t slot = abase + R.s * slot_bytes;
+                    uint64_t ad = swz_desc(slot, 64);
+                    uint64_t bd = swz_desc(g.resident ? rbase + b * g.b_bytes : slot + g.a_bytes, 64);
+                    for (int dy = 0; dy < 3; ++dy, ad += dy_a, bd += dy_b) {
 #pragma unroll
-                    for (int kk = 0; kk < KB / 16; ++kk)
-#pragma unroll
-                        for (int q = 0; q < MT; ++q)
-                            umma::mma_bf16(d + q * ncol, ad + (uint64_t)(q * (kBM * row / 16) + 2 * kk), bd + 2u * kk, idesc,
-                                           kk > 0 || add);
-                };
-                if constexpr (RES) {
-                    if (lane == 0) {
-                        const uint64_t bd = swz_desc(bbase + 3 * b * g.b_bytes, row);
-#pragma unroll
-                        for (int dy = 0; dy < 3; ++dy) issue(ad0 + dy * dy_a, bd + dy * (g.b_bytes >> 4), dy > 0 || b > 0);
+                        for (int kk = 0; kk < 2; ++kk)
+                            for (int q = 0; q < g.MT; ++q)
+                                umma::mma_bf16(d + q * ncol, ad + (uint64_t)(q * 512 + 2 * kk), bd + 2u * kk, idesc,
+                                               (b | dy | kk) != 0);
                     }
-                } else {
-#pragma unroll
-                    for (int dy = 0; dy < 3; ++dy) {
-                        ok = ok && mbar_wait_warp(&bfull[RB.s], RB.ph, g.err, kWaitNs);
-                        if (!ok) break;
-                        umma::tc_fence_after_sync();
-                        if (lane == 0) {
-                            issue(ad0 + dy * dy_a, swz_desc(bbase + RB.s * g.b_bytes, row), dy > 0 || b > 0);
-                            umma::mma_commit(&bempty[RB.s]);
-                        }
-                        __syncwarp();
-                        RB.next(g.bslots);
-                    }
+                    umma::mma_commit(&P.empty[R.s]);
                 }
-                if (!ok) break;
-                if (lane == 0) umma::mma_commit(&P.empty[R.s]);
                 __syncwarp();
                 R.next(g.slots);
             }
-            if (!ok) break;
             if (lane == 0) umma::mma_commit(&P.accf[a]);
             __syncwarp();
             done = tl + 1;
@@ -1050,14 +1006,13 @@ __global__ void __launch_bounds__(kRowThreads, 1)
         }
     } else {
         // ------------------------------------------------------------ epilogue
-        // two groups of four warps take the pixel tiles in turn, 32 channels at a time
+        // two groups of four warps take the 32-channel chunks in turn
         const int ew = warp & 3, eg = (warp - 2) >> 2;  // TMEM lane quarter of this warp, its group
         const uint32_t stage = sbase + (uint32_t)(warp - 2) * 4096u;
         const int x = (32 * ew + lane) & (g.W - 1);
         const bool first = x == 0, last = x == g.W - 1, cross = g.W > 32;
-        const bool wide = !g.f32 && g.ct == 64;  // staged and stored as 64 channels of bf16
         int buf = 0, par = 0;
-        uint32_t unit = 0;
+        uint32_t chunk = 0;
         for (int tl = 0; tl < ntl; ++tl) {
             const int a = g.nbuf == 2 ? tl & 1 : 0, use = g.nbuf == 2 ? tl >> 1 : tl;
             const bool ok = mbar_wait_warp(&P.accf[a], use & 1, g.err, kWaitNs);
@@ -1071,13 +1026,13 @@ __global__ void __launch_bounds__(kRowThreads, 1)
             umma::tc_fence_after_sync();
             if (!go) break;
             const int t = p0 + tl * pstep, img = t / g.ygroups, y0 = (t - img * g.ygroups) * g.rows;
-            for (int q = 0; q < MT; ++q) {
+            for (int q = 0; q < g.MT; ++q) {
                 if (y0 + q * (kBM / g.W) >= g.H) break;
-                if ((int)(unit++ & 1u) != eg) continue;
                 const int pix = (img * g.H + y0) * g.W + q * kBM + 32 * ew;  // of lane 0
                 for (int c0 = 0; c0 < g.ct; c0 += 32) {
+                    if ((int)(chunk++ & 1u) != eg) continue;
                     float v[32], l[32], r[32];
-                    const uint32_t col = P.taddr + ((uint32_t)(32 * ew) << 16) + (uint32_t)((a * MT + q) * ncol + c0);
+                    const uint32_t col = P.taddr + ((uint32_t)(32 * ew) << 16) + (uint32_t)((a * g.MT + q) * ncol + c0);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         umma::tmem_ld16(col + 16 * h, *reinterpret_cast<uint32_t(*)[16]>(l + 16 * h));
@@ -1105,15 +1060,15 @@ __global__ void __launch_bounds__(kRowThreads, 1)
                         if (g.relu) v[i] = fmaxf(v[i], 0.f);
                     }
                     par ^= 1;
-                    // staged as two chunks of 32 bf16, one of 64 or one of 32 fp32
-                    if (lane == 0 && !(wide && c0)) {
-                        if (g.f32 || wide)
+                    // staged as two chunks of bf16 or one of fp32
+                    if (lane == 0) {
+                        if (g.f32)
                             asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                         else
                             asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                     }
                     __syncwarp();
-                    const uint32_t dst = stage + (g.f32 || wide ? 0u : (uint32_t)buf * 2048u);
+                    const uint32_t dst = stage + (g.f32 ? 0u : (uint32_t)buf * 2048u);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {  // 8 channels
                         if (g.f32) {  // 128-byte rows, 128-byte swizzle
@@ -1124,7 +1079,7 @@ __global__ void __launch_bounds__(kRowThreads, 1)
                                              "f"(v[8 * j + 4 * h]), "f"(v[8 * j + 4 * h + 1]), "f"(v[8 * j + 4 * h + 2]),
                                              "f"(v[8 * j + 4 * h + 3])
                                              : "memory");
-                        } else {  // rows of 64 bytes, or of 128
+                        } else {  // 64-byte rows, 64-byte swizzle
                             uint32_t h[4];
 #pragma unroll
                             for (int i = 0; i < 4; ++i) {
@@ -1132,17 +1087,15 @@ __global__ void __launch_bounds__(kRowThreads, 1)
                                 h[i] = *reinterpret_cast<const uint32_t *>(&y);
                             }
                             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
-                                             dst + (uint32_t)(wide ? lane * 128 + (((c0 / 8 + j) ^ (lane & 7)) << 4)
-                                                        : lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4))),
+                                             dst + (uint32_t)(lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4))),
                                          "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3])
                                          : "memory");
                         }
                     }
-                    if (wide && !c0) continue;
                     umma::fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
-                        tma_store_2d(&omap, dst, nt * g.ct + (wide ? 0 : c0), pix);
+                        tma_store_2d(&omap, dst, nt * g.ct + c0, pix);
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
                     buf ^= 1;
@@ -2022,16 +1975,6 @@ int conv_tma(const agd_conv *c, const void *w, const float *bias, int relu, void
     return 1;
 }
 
-template <int KB, int MT, bool RES>
-int launch_row(const RowArgs &g, const CUtensorMap &xa0, const CUtensorMap &xa1, const CUtensorMap &wm,
-               const CUtensorMap &om, int blocks, int smem, cudaStream_t st) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(conv_row_kernel<KB, MT, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return set_cuda_error("conv3x3 shared memory", e);
-    conv_row_kernel<KB, MT, RES><<<blocks, kRowThreads, smem, st>>>(g, xa0, xa1, wm, om);
-    return launched("conv3x3 forward (rows)");
-}
-
 // The forward with the column taps side by side when the shapes allow it: 1
 // launched, 0 not applicable.  An M tile is 128 / W whole rows, channels move in
 // blocks of 32, and a channel tile is 64 (or 32) output channels.
@@ -2041,17 +1984,14 @@ int conv_row(const agd_conv *c, const void *w, const float *bias, int relu, void
     const bool two_in = s1.data != nullptr;
     void *out = out_bf16 ? out_bf16 : static_cast<void *>(out_f32);
     if (s0.up || (two_in && s1.up) || s0.channels % 32 || (two_in && s1.channels % 32) || c->cout % 32) return 0;
-    // few channels at 128 columns are conv_halo's: 32 -> 32 of 128 problems 90 us
-    // there against 138 here, 96 -> 32 233 us against 210
-    if (c->W == 128 && s0.channels + (two_in ? s1.channels : 0) < 96) return 0;
+    if (c->W == 128 && s0.channels + (two_in ? s1.channels : 0) < 96) return 0;  // conv_halo's: 90 us against 138 for 32 -> 32 channels (128 problems), 233 against 210 for 96 -> 32
     if (c->W < 8 || c->W > 128 || 128 % c->W || c->H % (128 / c->W) || reinterpret_cast<uintptr_t>(out) % 16) return 0;
     RowArgs g{};
     g.H = c->H;
     g.W = c->W;
-    g.kb = s0.channels % 64 || (two_in && s1.channels % 64) ? 32 : 64;
-    g.nblk0 = s0.channels / g.kb;
-    g.nblk = g.nblk0 + (two_in ? s1.channels / g.kb : 0);
-    g.cin = g.kb * g.nblk;
+    g.nblk0 = s0.channels / 32;
+    g.nblk = g.nblk0 + (two_in ? s1.channels / 32 : 0);
+    g.cin = 32 * g.nblk;
     g.N = c->cout;
     g.ct = c->cout % 64 ? 32 : 64;
     g.ntiles = c->cout / g.ct;
@@ -2063,20 +2003,16 @@ int conv_row(const agd_conv *c, const void *w, const float *bias, int relu, void
     if (M > 0x7fffffffLL) return 0;
     const int nsm = num_sms(), room = 227 * 1024 - 6144 - kRowStage;
     if (g.ntiles > nsm) return 0;
-    const int row = 2 * g.kb;
-    g.b_bytes = 3u * g.ct * row;
-    g.resident = 3LL * g.nblk * g.b_bytes <= 112 * 1024;
+    g.b_bytes = 9u * g.ct * 64u;
+    g.resident = (long long)g.nblk * g.b_bytes <= 112 * 1024;
     g.nbuf = g.resident || g.ct == 32 ? 2 : 1;
-    g.MT = std::min(2, 512 / (g.nbuf * 3 * g.ct));
+    g.MT = 512 / (g.nbuf * 3 * g.ct);
+    g.MT = g.MT >= 2 ? 2 : 1;
     while (true) {
         g.rows = g.MT * 128 / g.W;
-        g.a_bytes = (uint32_t)((g.rows + 2) * g.W * row);
-        g.bslots = g.resident ? 0 : 3;
-        g.slots = std::min(6, (room - (g.resident ? 3 * g.nblk : g.bslots) * (int)g.b_bytes) / (int)g.a_bytes);
-        if (g.slots == 1 && !g.resident) {
-            g.bslots = 2;
-            g.slots = (room - g.bslots * (int)g.b_bytes) / (int)g.a_bytes;
-        }
+        g.a_bytes = (uint32_t)(g.rows + 2) * g.W * 64u;  // a multiple of 512; slots on 1024 bytes below
+        const int slot = (int)((g.a_bytes + (g.resident ? 0u : g.b_bytes) + 1023u) / 1024u * 1024u);
+        g.slots = std::min(6, (room - (g.resident ? g.nblk * (int)g.b_bytes : 0)) / slot);
         if (g.slots >= 2 || g.MT == 1) break;
         g.MT = 1;
         g.nbuf = 2;
@@ -2091,26 +2027,26 @@ int conv_row(const agd_conv *c, const void *w, const float *bias, int relu, void
         const int C = sr.channels;
         const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)c->W, (cuuint64_t)c->H, (cuuint64_t)c->n};
         const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)c->W * C * 2, (cuuint64_t)c->H * c->W * C * 2};
-        const cuuint32_t box[4] = {(cuuint32_t)g.kb, (cuuint32_t)c->W, (cuuint32_t)(g.rows + 2), 1};
-        if (!make_map(k ? &xa1 : &xa0, sr.data, 4, dims, strides, box, row)) return 0;
+        const cuuint32_t box[4] = {32, (cuuint32_t)c->W, (cuuint32_t)(g.rows + 2), 1};
+        if (!make_map(k ? &xa1 : &xa0, sr.data, 4, dims, strides, box, 64)) return 0;
     }
     if (!two_in) xa1 = xa0;
     const cuuint64_t wdims[2] = {(cuuint64_t)kpad, (cuuint64_t)g.N}, wstr[1] = {(cuuint64_t)kpad * 2};
-    const cuuint32_t wbox[2] = {(cuuint32_t)g.kb, (cuuint32_t)g.ct};
+    const cuuint32_t wbox[2] = {32, (cuuint32_t)g.ct};
     const int esz = g.f32 ? 4 : 2;
     const cuuint64_t odims[2] = {(cuuint64_t)g.N, (cuuint64_t)M}, ostr[1] = {(cuuint64_t)g.N * esz};
-    const int och = !g.f32 && g.ct == 64 ? 64 : 32;
-    const cuuint32_t obox[2] = {(cuuint32_t)och, 32};
-    if (!make_map(&wm, w, 2, wdims, wstr, wbox, row) || !make_map(&om, out, 2, odims, ostr, obox, och * esz, g.f32)) return 0;
-    const int smem = 1024 + kRowStage + g.slots * (int)g.a_bytes + (g.resident ? 3 * g.nblk : g.bslots) * (int)g.b_bytes;
-    const int blocks = std::min(g.ptiles, std::max(1, nsm / g.ntiles)) * g.ntiles;
-    using Fn = int (*)(const RowArgs &, const CUtensorMap &, const CUtensorMap &, const CUtensorMap &, const CUtensorMap &,
-                       int, int, cudaStream_t);
-    static constexpr Fn fns[2][2][2] = {{{launch_row<32, 1, false>, launch_row<32, 1, true>},
-                                         {launch_row<32, 2, false>, launch_row<32, 2, true>}},
-                                        {{launch_row<64, 1, false>, launch_row<64, 1, true>},
-                                         {launch_row<64, 2, false>, launch_row<64, 2, true>}}};
-    *rc = fns[g.kb == 64][g.MT == 2][g.resident](g, xa0, xa1, wm, om, blocks, smem, st);
+    const cuuint32_t obox[2] = {32, 32};
+    if (!make_map(&wm, w, 2, wdims, wstr, wbox, 64) || !make_map(&om, out, 2, odims, ostr, obox, 32 * esz, g.f32)) return 0;
+    const int smem = 1024 + kRowStage + g.slots * (int)(g.a_bytes + (g.resident ? 0u : g.b_bytes)) +
+                     (g.resident ? g.nblk * (int)g.b_bytes : 0);
+    const cudaError_t e = cudaFuncSetAttribute(conv_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+        *rc = set_cuda_error("conv3x3 shared memory", e);
+        return 1;
+    }
+    const int groups = std::min(g.ptiles, std::max(1, nsm / g.ntiles));
+    conv_row_kernel<<<groups * g.ntiles, kRowThreads, smem, st>>>(g, xa0, xa1, wm, om);
+    *rc = launched("conv3x3 forward (rows)");
     return 1;
 }
 
