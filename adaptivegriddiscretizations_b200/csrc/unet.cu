@@ -859,263 +859,6 @@ __global__ void __launch_bounds__(kHaloThreads, 1)
     }
 }
 
-// ------------------------------------ forward with the column taps side by side
-// The same GEMM for images of W | 128 columns: what bounds an MMA of 128 pixels
-// and few channels is the reading of its A operand, 64 cycles per 128 x 16 whatever
-// N is up to 128.  So the three column taps dx share it: N = 3 x ct columns (dx,
-// channel), K = (dy, input channel), D[p, (dx, co)] = sum X[p + dy W, ci] w[co, dy, dx, ci],
-// and the epilogue forms out[p] = D[p - 1, 0] + D[p, 1] + D[p + 1, 2], zero beyond a
-// row's ends (shuffles between the lanes, which are the pixels, and shared
-// memory between the warps).  A CTA tile is MT x 128 pixels, whole rows; per
-// block of 32 channels one copy brings its rows and one above and below, and the
-// row taps dy are the same data W pixel rows further on, whole swizzle atoms.
-// Weights stay resident where they fit (they are then loaded once a CTA; with
-// several channel tiles, a CTA keeps to one of them), else they come with each block.
-// Accumulators: double buffered, or two pixel tiles at once where the weights
-// are not resident, so that a block of them serves 256 pixels.
-// Measured (128 problems): the 12 layers at 64^2 and below and the 96 -> 32 one at 128^2
-// 1475 -> 920 us, the forward 1.99 -> 1.31 ms.
-constexpr int kRowThreads = 320;   // a producer, an MMA and 2 x 4 epilogue warps
-constexpr int kRowStage = 32768;   // staging of the epilogue: 8 warps x 4 KB
-
-struct RowArgs {
-    int H, W, rows;      // rows of a CTA tile (MT 128 / W)
-    int nblk0, nblk;     // 32-channel blocks of the first input, of both
-    int cin, ct, ntiles; // input channels, output channels of a tile, channel tiles
-    int MT, nbuf, resident, slots;
-    int ygroups, ptiles; // row groups of an image, pixel tiles of the launch
-    uint32_t a_bytes, b_bytes;  // a slot's rows, and the weights of a block (3 dy)
-    const float *bias;
-    int relu, f32, N;
-    unsigned *err;
-};
-
-__global__ void __launch_bounds__(kRowThreads, 1)
-    conv_row_kernel(RowArgs g, const __grid_constant__ CUtensorMap xa0, const __grid_constant__ CUtensorMap xa1,
-                    const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap omap) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ HaloPipe P;
-    __shared__ float edge[2][2][4][2][32];  // by group, parity of its chunk, warp: last pixel's D0 and first pixel's D2
-    __shared__ __align__(16) float sbias[64];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t sbase = (umma::smem_u32(smem) + 1023u) & ~1023u;
-    const uint32_t abase = sbase + kRowStage;
-    const uint32_t slot_bytes = g.a_bytes + (g.resident ? 0u : g.b_bytes);
-    const uint32_t rbase = abase + g.slots * slot_bytes;  // resident weights
-    const int ncol = 3 * g.ct;                            // accumulator columns of a pixel tile
-    const uint32_t tcols = tmem_cols(g.nbuf * g.MT * ncol);
-    // CTA c works on channel tile c % ntiles and every (grid / ntiles)-th pixel tile
-    const int nt = blockIdx.x % g.ntiles, p0 = blockIdx.x / g.ntiles, pstep = gridDim.x / g.ntiles;
-    const int ntl = p0 < g.ptiles && p0 < pstep ? (g.ptiles - p0 + pstep - 1) / pstep : 0;
-
-    if (warp == 1) {
-        umma::tmem_alloc(&P.taddr, tcols);
-        umma::tmem_relinquish();
-    }
-    if (tid == 0) {
-        for (int s = 0; s < g.slots; ++s) {
-            umma::mbar_init(&P.full[s], 1);
-            umma::mbar_init(&P.empty[s], 1);
-        }
-        for (int a = 0; a < 2; ++a) {
-            umma::mbar_init(&P.accf[a], 1);
-            umma::mbar_init(&P.acce[a], 8);
-        }
-        umma::mbar_init(&P.bready, 1);
-        umma::fence_mbar_init();
-    }
-    if (tid < g.ct) sbias[tid] = g.bias ? __ldg(g.bias + nt * g.ct + tid) : 0.f;
-    umma::tc_fence_before_sync();
-    __syncthreads();
-    umma::tc_fence_after_sync();
-
-    if (warp == 0) {
-        // ------------------------------------------------------------ producer
-        // the weights of block b: for each dy the rows (dx, channel) of 64 bytes
-        auto load_weights = [&](uint32_t dst, int b, uint64_t *bar) {
-            for (int tap = 0; tap < 9; ++tap)
-                tma_load_2d(dst + (uint32_t)(tap * g.ct) * 64u, &wmap, tap * g.cin + 32 * b, nt * g.ct, bar);
-        };
-        if (lane == 0 && g.resident && ntl > 0) {
-            mbar_expect_tx(&P.bready, (uint32_t)g.nblk * g.b_bytes);
-            for (int b = 0; b < g.nblk; ++b) load_weights(rbase + b * g.b_bytes, b, &P.bready);
-        }
-        __syncwarp();
-        Ring R;
-        bool wrapped = false, alive = true;
-        for (int tl = 0; tl < ntl && alive; ++tl) {
-            const int t = p0 + tl * pstep, img = t / g.ygroups, y0 = (t - img * g.ygroups) * g.rows;
-            for (int b = 0; b < g.nblk; ++b) {
-                if (wrapped && !mbar_wait_warp(&P.empty[R.s], R.ph ^ 1u, g.err, kWaitNs)) {
-                    alive = false;
-                    break;
-                }
-                if (lane == 0) {
-                    const uint32_t slot = abase + R.s * slot_bytes;
-                    mbar_expect_tx(&P.full[R.s], slot_bytes);
-                    tma_load_4d(slot, b < g.nblk0 ? &xa0 : &xa1, 32 * (b < g.nblk0 ? b : b - g.nblk0), 0, y0 - 1, img,
-                                &P.full[R.s]);
-                    if (!g.resident) load_weights(slot + g.a_bytes, b, &P.full[R.s]);
-                }
-                __syncwarp();
-                R.next(g.slots);
-                wrapped = wrapped || R.s == 0;
-            }
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------ MMA (lane 0 issues)
-        const uint32_t idesc = umma::idesc_bf16(kBM, ncol, 0, 0);
-        const uint64_t dy_a = (uint64_t)((uint32_t)g.W * 64u >> 4), dy_b = (uint64_t)((uint32_t)ncol * 64u >> 4);
-        Ring R;
-        bool ok = ntl > 0 && (!g.resident || mbar_wait_warp(&P.bready, 0, g.err, kWaitNs));
-        int done = 0;
-        for (int tl = 0; tl < ntl && ok; ++tl) {
-            const int a = g.nbuf == 2 ? tl & 1 : 0, use = g.nbuf == 2 ? tl >> 1 : tl;  // the buffer's use-th tile
-            if (use > 0 && !mbar_wait_warp(&P.acce[a], (use & 1) ^ 1, g.err, kWaitNs)) break;
-            umma::tc_fence_after_sync();
-            const uint32_t d = P.taddr + (uint32_t)(a * g.MT * ncol);
-            for (int b = 0; b < g.nblk; ++b) {
-                if (!mbar_wait_warp(&P.full[R.s], R.ph, g.err, kWaitNs)) {
-                    ok = false;
-                    break;
-                }
-                umma::tc_fence_after_sync();
-                if (lane == 0) {
-                    const uint32_t slot = abase + R.s * slot_bytes;
-                    uint64_t ad = swz_desc(slot, 64);
-                    uint64_t bd = swz_desc(g.resident ? rbase + b * g.b_bytes : slot + g.a_bytes, 64);
-                    for (int dy = 0; dy < 3; ++dy, ad += dy_a, bd += dy_b) {
-#pragma unroll
-                        for (int kk = 0; kk < 2; ++kk)
-                            for (int q = 0; q < g.MT; ++q)
-                                umma::mma_bf16(d + q * ncol, ad + (uint64_t)(q * 512 + 2 * kk), bd + 2u * kk, idesc,
-                                               (b | dy | kk) != 0);
-                    }
-                    umma::mma_commit(&P.empty[R.s]);
-                }
-                __syncwarp();
-                R.next(g.slots);
-            }
-            if (lane == 0) umma::mma_commit(&P.accf[a]);
-            __syncwarp();
-            done = tl + 1;
-        }
-        if (done > 0) {
-            const int a = g.nbuf == 2 ? (done - 1) & 1 : 0, use = g.nbuf == 2 ? (done - 1) >> 1 : done - 1;
-            mbar_wait_warp(&P.accf[a], use & 1, g.err, kWaitNs);
-        }
-    } else {
-        // ------------------------------------------------------------ epilogue
-        // two groups of four warps take the 32-channel chunks in turn
-        const int ew = warp & 3, eg = (warp - 2) >> 2;  // TMEM lane quarter of this warp, its group
-        const uint32_t stage = sbase + (uint32_t)(warp - 2) * 4096u;
-        const int x = (32 * ew + lane) & (g.W - 1);
-        const bool first = x == 0, last = x == g.W - 1, cross = g.W > 32;
-        int buf = 0, par = 0;
-        uint32_t chunk = 0;
-        for (int tl = 0; tl < ntl; ++tl) {
-            const int a = g.nbuf == 2 ? tl & 1 : 0, use = g.nbuf == 2 ? tl >> 1 : tl;
-            const bool ok = mbar_wait_warp(&P.accf[a], use & 1, g.err, kWaitNs);
-            int go;
-            // the four warps of a group leave together (they share barriers below)
-            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\t"
-                         "barrier.cta.red.and.pred q, %2, 128, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
-                         : "=r"(go)
-                         : "r"((int)ok), "r"(1 + 2 * eg)
-                         : "memory");
-            umma::tc_fence_after_sync();
-            if (!go) break;
-            const int t = p0 + tl * pstep, img = t / g.ygroups, y0 = (t - img * g.ygroups) * g.rows;
-            for (int q = 0; q < g.MT; ++q) {
-                if (y0 + q * (kBM / g.W) >= g.H) break;
-                const int pix = (img * g.H + y0) * g.W + q * kBM + 32 * ew;  // of lane 0
-                for (int c0 = 0; c0 < g.ct; c0 += 32) {
-                    if ((int)(chunk++ & 1u) != eg) continue;
-                    float v[32], l[32], r[32];
-                    const uint32_t col = P.taddr + ((uint32_t)(32 * ew) << 16) + (uint32_t)((a * g.MT + q) * ncol + c0);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        umma::tmem_ld16(col + 16 * h, *reinterpret_cast<uint32_t(*)[16]>(l + 16 * h));
-                        umma::tmem_ld16(col + g.ct + 16 * h, *reinterpret_cast<uint32_t(*)[16]>(v + 16 * h));
-                        umma::tmem_ld16(col + 2 * g.ct + 16 * h, *reinterpret_cast<uint32_t(*)[16]>(r + 16 * h));
-                    }
-                    umma::tmem_ld_wait();
-                    if (cross) {  // neighbours of another warp
-                        if (lane == 31)
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) edge[eg][par][ew][0][i] = l[i];
-                        if (lane == 0)
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) edge[eg][par][ew][1][i] = r[i];
-                        asm volatile("barrier.cta.sync %0, 128;" ::"r"(2 + 2 * eg) : "memory");
-                    }
-                    const float *el = edge[eg][par][(ew + 3) & 3][0], *er = edge[eg][par][(ew + 1) & 3][1];
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        float a0 = __shfl_up_sync(0xffffffffu, l[i], 1), a2 = __shfl_down_sync(0xffffffffu, r[i], 1);
-                        if (cross && lane == 0) a0 = el[i];
-                        if (cross && lane == 31) a2 = er[i];
-                        v[i] += (first ? 0.f : a0) + (last ? 0.f : a2);
-                        v[i] += sbias[c0 + i];
-                        if (g.relu) v[i] = fmaxf(v[i], 0.f);
-                    }
-                    par ^= 1;
-                    // staged as two chunks of bf16 or one of fp32
-                    if (lane == 0) {
-                        if (g.f32)
-                            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                        else
-                            asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                    }
-                    __syncwarp();
-                    const uint32_t dst = stage + (g.f32 ? 0u : (uint32_t)buf * 2048u);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {  // 8 channels
-                        if (g.f32) {  // 128-byte rows, 128-byte swizzle
-#pragma unroll
-                            for (int h = 0; h < 2; ++h)
-                                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(
-                                                 dst + (uint32_t)(lane * 128 + (((2 * j + h) ^ (lane & 7)) << 4))),
-                                             "f"(v[8 * j + 4 * h]), "f"(v[8 * j + 4 * h + 1]), "f"(v[8 * j + 4 * h + 2]),
-                                             "f"(v[8 * j + 4 * h + 3])
-                                             : "memory");
-                        } else {  // 64-byte rows, 64-byte swizzle
-                            uint32_t h[4];
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const __nv_bfloat162 y = __floats2bfloat162_rn(v[8 * j + 2 * i], v[8 * j + 2 * i + 1]);
-                                h[i] = *reinterpret_cast<const uint32_t *>(&y);
-                            }
-                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
-                                             dst + (uint32_t)(lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4))),
-                                         "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3])
-                                         : "memory");
-                        }
-                    }
-                    umma::fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-                        tma_store_2d(&omap, dst, nt * g.ct + c0, pix);
-                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    }
-                    buf ^= 1;
-                }
-            }
-            umma::tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(&P.acce[a])) : "memory");
-        }
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-        __syncwarp();
-    }
-    umma::tc_fence_before_sync();
-    __syncthreads();
-    if (warp == 1) {
-        umma::tc_fence_after_sync();
-        umma::tmem_dealloc(P.taddr, tcols);
-    }
-}
-
 // Weight gradient: dW[n, r] += sum_p dZ[p, n] X[p + tap(r), ci(r)], r = tap *
 // cin + ci.  GEMM with M = r (128 per tile), N = n, K = pixels (64 per stage,
 // split over `splits` work items): both operands MN-major (8 consecutive
@@ -1394,23 +1137,18 @@ __global__ void avgpool_kernel(const bf16 *x, int n, int H, int W, int C, bf16 *
     *reinterpret_cast<uint4 *>(y + p * C + c8 * 8) = w;
 }
 
-// Nearest 2x upsampling, NHWC bf16 (n, H, W, C) -> (n, 2H, 2W, C): a thread reads
-// 8 channels of an input pixel once and writes them to its four output pixels.
-// Bound by the writes; I is 32 bits where the input has less than 2^31 vectors
-// (64-bit divisions, and a thread per output vector, took 99 us instead of
-// 50 us for 128 x 64 x 64 x 64).
-template <class I>
-__global__ void upsample_kernel(const bf16 *x, I m, I W, I C8, bf16 *y) {
-    const I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
-    if (idx >= m) return;
-    const I p = idx / C8, c8 = idx - p * C8, row = p / W, ix = p - row * W;  // row: of all images
-    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(x) + idx);
-    const long long pitch = 2LL * W * C8;
-    uint4 *o = reinterpret_cast<uint4 *>(y) + 2LL * row * pitch + 2LL * ix * C8 + c8;
-    o[0] = v;
-    o[C8] = v;
-    o[pitch] = v;
-    o[pitch + C8] = v;
+// Nearest 2x upsampling, NHWC bf16 (n, H, W, C) -> (n, 2H, 2W, C), 8 channels per thread.
+__global__ void upsample_kernel(const bf16 *x, int n, int H, int W, int C, bf16 *y) {
+    const int C8 = C / 8;
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long long)n * 4 * H * W * C8) return;
+    const int c8 = (int)(idx % C8);
+    const long long p = idx / C8;  // output pixel
+    const int b = (int)(p / (4LL * H * W));
+    const int r = (int)(p - (long long)b * 4 * H * W);
+    const int oy = r / (2 * W), ox = r - (r / (2 * W)) * (2 * W);
+    *reinterpret_cast<uint4 *>(y + p * C + c8 * 8) =
+        *reinterpret_cast<const uint4 *>(x + (((long long)b * H + oy / 2) * W + ox / 2) * C + c8 * 8);
 }
 
 // Backward routing into a layer output Y (n, H, W, C): the gradient of Y is the
@@ -1975,81 +1713,6 @@ int conv_tma(const agd_conv *c, const void *w, const float *bias, int relu, void
     return 1;
 }
 
-// The forward with the column taps side by side when the shapes allow it: 1
-// launched, 0 not applicable.  An M tile is 128 / W whole rows, channels move in
-// blocks of 32, and a channel tile is 64 (or 32) output channels.
-int conv_row(const agd_conv *c, const void *w, const float *bias, int relu, void *out_bf16, float *out_f32,
-             unsigned *err, cudaStream_t st, int *rc) {
-    const agd_conv_src &s0 = c->src[0], &s1 = c->src[1];
-    const bool two_in = s1.data != nullptr;
-    void *out = out_bf16 ? out_bf16 : static_cast<void *>(out_f32);
-    if (s0.up || (two_in && s1.up) || s0.channels % 32 || (two_in && s1.channels % 32) || c->cout % 32) return 0;
-    if (c->W == 128 && s0.channels + (two_in ? s1.channels : 0) < 96) return 0;  // conv_halo's: 90 us against 138 for 32 -> 32 channels (128 problems), 233 against 210 for 96 -> 32
-    if (c->W < 8 || c->W > 128 || 128 % c->W || c->H % (128 / c->W) || reinterpret_cast<uintptr_t>(out) % 16) return 0;
-    RowArgs g{};
-    g.H = c->H;
-    g.W = c->W;
-    g.nblk0 = s0.channels / 32;
-    g.nblk = g.nblk0 + (two_in ? s1.channels / 32 : 0);
-    g.cin = 32 * g.nblk;
-    g.N = c->cout;
-    g.ct = c->cout % 64 ? 32 : 64;
-    g.ntiles = c->cout / g.ct;
-    g.bias = bias;
-    g.relu = relu;
-    g.f32 = out_f32 != nullptr;
-    g.err = err;
-    const long long M = (long long)c->n * c->H * c->W;
-    if (M > 0x7fffffffLL) return 0;
-    const int nsm = num_sms(), room = 227 * 1024 - 6144 - kRowStage;
-    if (g.ntiles > nsm) return 0;
-    g.b_bytes = 9u * g.ct * 64u;
-    g.resident = (long long)g.nblk * g.b_bytes <= 112 * 1024;
-    g.nbuf = g.resident || g.ct == 32 ? 2 : 1;
-    g.MT = 512 / (g.nbuf * 3 * g.ct);
-    g.MT = g.MT >= 2 ? 2 : 1;
-    while (true) {
-        g.rows = g.MT * 128 / g.W;
-        g.a_bytes = (uint32_t)(g.rows + 2) * g.W * 64u;  // a multiple of 512; slots on 1024 bytes below
-        const int slot = (int)((g.a_bytes + (g.resident ? 0u : g.b_bytes) + 1023u) / 1024u * 1024u);
-        g.slots = std::min(6, (room - (g.resident ? g.nblk * (int)g.b_bytes : 0)) / slot);
-        if (g.slots >= 2 || g.MT == 1) break;
-        g.MT = 1;
-        g.nbuf = 2;
-    }
-    if (g.slots < 2 || g.a_bytes % 1024 || g.b_bytes % 1024) return 0;
-    g.ygroups = (c->H + g.rows - 1) / g.rows;
-    g.ptiles = c->n * g.ygroups;
-    const int kpad = kpad_of(9 * g.cin);
-    CUtensorMap xa0, xa1, wm, om;
-    for (int k = 0; k < (two_in ? 2 : 1); ++k) {
-        const agd_conv_src &sr = c->src[k];
-        const int C = sr.channels;
-        const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)c->W, (cuuint64_t)c->H, (cuuint64_t)c->n};
-        const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)c->W * C * 2, (cuuint64_t)c->H * c->W * C * 2};
-        const cuuint32_t box[4] = {32, (cuuint32_t)c->W, (cuuint32_t)(g.rows + 2), 1};
-        if (!make_map(k ? &xa1 : &xa0, sr.data, 4, dims, strides, box, 64)) return 0;
-    }
-    if (!two_in) xa1 = xa0;
-    const cuuint64_t wdims[2] = {(cuuint64_t)kpad, (cuuint64_t)g.N}, wstr[1] = {(cuuint64_t)kpad * 2};
-    const cuuint32_t wbox[2] = {32, (cuuint32_t)g.ct};
-    const int esz = g.f32 ? 4 : 2;
-    const cuuint64_t odims[2] = {(cuuint64_t)g.N, (cuuint64_t)M}, ostr[1] = {(cuuint64_t)g.N * esz};
-    const cuuint32_t obox[2] = {32, 32};
-    if (!make_map(&wm, w, 2, wdims, wstr, wbox, 64) || !make_map(&om, out, 2, odims, ostr, obox, 32 * esz, g.f32)) return 0;
-    const int smem = 1024 + kRowStage + g.slots * (int)(g.a_bytes + (g.resident ? 0u : g.b_bytes)) +
-                     (g.resident ? g.nblk * (int)g.b_bytes : 0);
-    const cudaError_t e = cudaFuncSetAttribute(conv_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-        *rc = set_cuda_error("conv3x3 shared memory", e);
-        return 1;
-    }
-    const int groups = std::min(g.ptiles, std::max(1, nsm / g.ntiles));
-    conv_row_kernel<<<groups * g.ntiles, kRowThreads, smem, st>>>(g, xa0, xa1, wm, om);
-    *rc = launched("conv3x3 forward (rows)");
-    return 1;
-}
-
 }  // namespace
 
 extern "C" {
@@ -2063,8 +1726,6 @@ int agd_conv3x3_forward(const agd_conv *c, const void *w, const float *bias, int
     if (!w || !err || (!out_bf16) == (!out_f32) || c->cout <= 0 || c->cout % 16)
         return set_error(AGD_STATUS_INVALID, "conv3x3: weights, err, one output and cout % 16 == 0 are required");
     int rc = AGD_STATUS_OK;
-    if (reinterpret_cast<uintptr_t>(w) % 16 == 0 && conv_row(c, w, bias, relu, out_bf16, out_f32, err, cs(stream), &rc))
-        return rc;
     if (reinterpret_cast<uintptr_t>(w) % 16 == 0 && conv_halo(c, w, bias, relu, out_bf16, out_f32, err, cs(stream), &rc))
         return rc;
     if (reinterpret_cast<uintptr_t>(w) % 16 == 0 && conv_tma(c, w, bias, relu, out_bf16, out_f32, err, cs(stream), &rc))
@@ -2181,14 +1842,9 @@ int agd_ws_avgpool(const void *x, int n, int H, int W, int C, void *y, agd_strea
 
 int agd_ws_upsample(const void *x, int n, int H, int W, int C, void *y, agd_stream_t stream) {
     if (!x || !y || n <= 0 || H <= 0 || W <= 0 || C % 8) return set_error(AGD_STATUS_INVALID, "upsample: bad arguments");
-    const long long m = (long long)n * H * W * (C / 8);
-    const unsigned blocks = (unsigned)((m + 255) / 256);
-    if (m < 0x7fffff00LL)
-        upsample_kernel<unsigned><<<blocks, 256, 0, cs(stream)>>>(static_cast<const bf16 *>(x), (unsigned)m, (unsigned)W,
-                                                                  (unsigned)(C / 8), static_cast<bf16 *>(y));
-    else
-        upsample_kernel<long long><<<blocks, 256, 0, cs(stream)>>>(static_cast<const bf16 *>(x), m, (long long)W,
-                                                                   (long long)(C / 8), static_cast<bf16 *>(y));
+    const long long m = (long long)n * 4 * H * W * (C / 8);
+    upsample_kernel<<<(unsigned)((m + 255) / 256), 256, 0, cs(stream)>>>(static_cast<const bf16 *>(x), n, H, W, C,
+                                                                         static_cast<bf16 *>(y));
     return launched("upsample");
 }
 
