@@ -124,3 +124,38 @@ def test_reverse_with_a_cycle():
     assert int(stats[0].item()) >> 32 == 0
     # 200 steps, each passing changes above 5e-6 of the value on
     assert np.abs(lam.cpu().numpy() - ref).max() <= 2e-5 * np.abs(ref).max()
+
+
+def test_rounds_captured_and_two_streams():
+    """The rounds' cooperative launch in a captured graph, replayed, and two solves in flight
+    on two streams: the values are the plain run's (the schedule may differ: within tolerance)."""
+    from adaptivegriddiscretizations_b200.Eikonal.HFM_CUDA import BatchPlan
+    cases = [_case("Riemann2", (163, 129), 5), _case("Isotropic2", (130, 257), 6)]
+    itfs = _interfaces(cases)
+    plans = [BatchPlan([it]) for it in itfs]
+
+    def step(k):
+        itfs[k].values_t.fill_(float("inf"))
+        plans[k].run()
+
+    streams = [torch.cuda.Stream() for _ in plans]
+    for _ in range(3):
+        for k, s in enumerate(streams):
+            s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(s):
+                step(k)
+    torch.cuda.synchronize()
+    for it, c in zip(itfs, cases):
+        _close(it.squeeze(it.values_t).cpu().numpy(), c)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for k in range(2):
+            step(k)
+    for it in itfs:
+        it.values_t.zero_()
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    for p, it, c in zip(plans, itfs, cases):
+        assert not p.read_stats()[1].any()
+        _close(it.squeeze(it.values_t).cpu().numpy(), c)
